@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include "direct.h"
 #include "engine.h"
 
 namespace brig {
@@ -286,7 +287,13 @@ int64_t Engine::workspace_needed(const brig_join_config& cfg, const std::vector<
     std::vector<JoinOffs> jo(plans.size());
     Shape sh;
     layout_for(cfg, plans.data(), (int)plans.size(), num_sms, jo.data(), sh);
-    return (int64_t)sh.total;
+    size_t total = sh.total;
+    if (plans.size() == 1 && direct_eligible(cfg, plans[0])) {
+        DirectShape ds;
+        direct_layout(plans[0], 2 * num_sms, ds);
+        total = std::max(total, ds.total);
+    }
+    return (int64_t)total;
 }
 
 Engine::Engine(const brig_join_config& cfg) : cfg_(cfg) {
@@ -678,6 +685,45 @@ void fill_pipeline(const brig_join_config& cfg, const JoinPlan* plans, const Joi
     }
 }
 
+void Engine::finish_run(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, int64_t* counters,
+                        unsigned long long* gwords, cudaStream_t stream) {
+    const int nj = (int)joins.size();
+    note_survivors(plans, counters, stream);
+    cuda_check(cudaEventRecord(done_, stream), "cudaEventRecord");
+    have_run_ = true;
+    if (profiling_) ++runs_recorded_;
+    plans_ = plans;
+    caps_.resize(nj);
+    for (int j = 0; j < nj; ++j) caps_[j] = joins[j].out.capacity;
+    d_counters_ = counters;
+    d_gwords_ = gwords;
+    nj_ = nj;
+}
+
+void Engine::run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream) {
+    const JoinPlan& p = plans[0];
+    int& per_sm = direct_ctas_[!p.bloom ? 0 : 1 + 2 * (p.pf.mode != 0) + (p.k == kBloomFastK)];
+    if (!per_sm) {
+        cuda_check(direct_residency(p.bloom, p.pf.mode, p.k, &per_sm), "direct join residency");
+        per_sm = std::min(std::max(per_sm, 1), 2);
+    }
+    DirectShape sh;
+    direct_layout(p, per_sm * num_sms_, sh);
+    if (have_run_) cuda_check(cudaStreamWaitEvent(stream, done_, 0), "cudaStreamWaitEvent");
+    ensure_workspace(sh.total, stream);
+    DirectArgs a;
+    direct_fill(p, joins[0], sh, ws_, a);
+    int64_t* counters = reinterpret_cast<int64_t*>(ws_ + sh.counters);
+    cudaEvent_t* ev = profiling_ ? stage_ev_[runs_recorded_ % kStageRing] : nullptr;
+    // the whole join is one kernel: its time shows as the last stage
+    for (int i = 0; ev && i < kNumStages; ++i) cuda_check(cudaEventRecord(ev[i], stream), "cudaEventRecord");
+    // the counters and the state words are adjacent
+    cuda_check(cudaMemsetAsync(counters, 0, sh.gwords + kDirectWords * 8 - sh.counters, stream), "state reset");
+    cuda_check(enqueue_direct(a, p.bloom, p.pf.mode, p.k, sh.grid, stream), "direct join launch");
+    if (ev) cuda_check(cudaEventRecord(ev[kNumStages], stream), "cudaEventRecord");
+    finish_run(joins, plans, counters, a.gwords, stream);
+}
+
 void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use_graph, cudaEvent_t s_ready) {
     if (s_ready) use_graph = false;
     const int nj = (int)joins.size();
@@ -688,6 +734,12 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
         ns[j] = joins[j].ns;
     }
     std::vector<JoinPlan> plans = plan_batch(adapt_config(nj), nr.data(), ns.data(), nj, shared_l2_);
+    // A direct join is one kernel whose descriptor is its argument, so a graph would save it nothing.
+    if (nj == 1 && direct_eligible(cfg_, plans[0])) {
+        if (s_ready) cuda_check(cudaStreamWaitEvent(stream, s_ready, 0), "cudaStreamWaitEvent");
+        run_direct(joins, plans, stream);
+        return;
+    }
     std::vector<JoinOffs> jo(nj);
     Shape sh;
     layout_for(cfg_, plans.data(), nj, num_sms_, jo.data(), sh);
@@ -743,7 +795,7 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
                 graph_exec_ = nullptr;
             }
             // Kernel attributes are set on the first direct launch, outside capture.
-            if (!have_run_) {
+            if (!pipeline_loaded_) {
                 enqueue_all(stream);
                 cuda_check(cudaStreamSynchronize(stream), "warm-up run");
             }
@@ -775,16 +827,8 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
         enqueue_all(stream);
     }
     if (use_graph) cuda_check(cudaEventRecord(stage_free_, stream), "cudaEventRecord");
-    note_survivors(plans, counters, stream);
-    cuda_check(cudaEventRecord(done_, stream), "cudaEventRecord");
-    have_run_ = true;
-    if (profiling_) ++runs_recorded_;
-    plans_ = plans;
-    caps_.resize(nj);
-    for (int j = 0; j < nj; ++j) caps_[j] = joins[j].out.capacity;
-    d_counters_ = counters;
-    d_gwords_ = a.gwords;
-    nj_ = nj;
+    pipeline_loaded_ = true;
+    finish_run(joins, plans, counters, a.gwords, stream);
 }
 
 // The adaptive filter's break-even: at |R| = 2^26, |S| = 2^30 and 10 bits/key the filtered join

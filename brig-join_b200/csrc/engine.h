@@ -170,6 +170,10 @@ public:
                           cudaStream_t stream);
 
 private:
+    // The unpartitioned join (direct.cu) of a join that direct_eligible accepts.
+    void run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream);
+    void finish_run(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, int64_t* counters,
+                    unsigned long long* gwords, cudaStream_t stream);
     void ensure_workspace(size_t bytes, cudaStream_t stream);
     void ensure_staging(size_t bytes);
 
@@ -183,6 +187,8 @@ private:
     cudaEvent_t stage_free_ = nullptr;  // recorded after the staging copy
     cudaEvent_t done_ = nullptr;        // recorded after the last run
     bool have_run_ = false;
+    bool pipeline_loaded_ = false;   // the partitioned pipeline has run on this handle
+    int direct_ctas_[5] = {};        // CTAs per SM of the unpartitioned join's kernels (0: not asked yet)
     bool shared_l2_ = false;
     std::vector<JoinPlan> plans_;
     std::vector<int64_t> caps_;

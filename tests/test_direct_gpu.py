@@ -1,0 +1,81 @@
+"""The unpartitioned join (one cooperative kernel) against the oracle and the partitioned join: step and
+tile remainders, both build sides, long buckets, the limits of the rule that chooses it."""
+import numpy as np
+import pytest
+
+from gpu_helpers import assert_same_pairs, run_device
+
+pytestmark = pytest.mark.gpu
+MAX_BUILD = 3 << 20
+
+
+def _join(bj, oracle, torch, data, launches=1, **cfg):
+    exp = oracle.pairs(*data)
+    n0 = bj.kernel_launches()
+    st, r, s, k = run_device(bj, torch, *data, cap=max(len(exp[0]), 1), **cfg)
+    if launches:
+        assert bj.kernel_launches() - n0 == launches  # the path under test ran
+    assert st.count == len(exp[0])
+    assert_same_pairs(oracle, r, s, *exp)
+    if k is not None:
+        key = dict(zip(data[3].tolist(), data[2].tolist()))
+        assert all(key[v] == q for v, q in zip(s.tolist(), k.tolist()))
+    return st
+
+
+@pytest.mark.parametrize("n_r,n_s", [(1, 1), (1, 4096), (127, 129), (3275, 3277), (4097, 65_537), (65_537, 4097),
+                                     (200_003, 1_000_001), (1_000_001, 300_007)])
+@pytest.mark.parametrize("cfg", [dict(), dict(use_bloom=1), dict(use_bloom=1, bloom_bits_per_key=14.0),
+                                 dict(use_bloom=1, partition_mode=1)], ids=["plain", "k7", "k10", "modulo"])
+def test_sizes(bj, oracle, torch_cuda, n_r, n_s, cfg):
+    st = _join(bj, oracle, torch_cuda, bj.gen_host(n_r + n_s, n_r, n_s, 0.3), **cfg)
+    if not cfg:
+        assert st.s_survivors == n_s
+    else:  # the same filter as the partitioned join's: the same survivors
+        p = run_device(bj, torch_cuda, *bj.gen_host(n_r + n_s, n_r, n_s, 0.3), partition_size=st.partition_size,
+                       second_partition_size=st.second_partition_size, **cfg)[0]
+        assert (st.s_survivors, st.bloom_num_bits) == (p.s_survivors, p.bloom_num_bits)
+
+
+@pytest.mark.parametrize("bloom", [0, 1])
+@pytest.mark.parametrize("build", ["r", "s"])
+@pytest.mark.parametrize("copies", [2, 9, 10, 254, 255, 256, 700, 20_000])
+def test_repeated_build_keys(bj, oracle, torch_cuda, copies, build, bloom):
+    """Buckets at the edges of the lock-step walk (8), the counted length (255) and the listed pieces (256)."""
+    rng = np.random.default_rng(copies)
+    hot = np.repeat(np.array([7, 0x80000000, 0xFFFFFFFF], np.uint32), [copies, max(copies // 2, 1), 3])
+    small = rng.permutation(np.concatenate([hot, np.arange(100, 20_100, dtype=np.uint32)]))
+    big = rng.permutation(np.concatenate([np.arange(10_000, 60_000, dtype=np.uint32),
+                                          np.array([7, 7, 0x80000000, 0xFFFFFFFF, 5], np.uint32)]))
+    rk, sk = (small, big) if build == "r" else (big, small)
+    data = (rk, np.arange(len(rk), dtype=np.uint32), sk, np.arange(len(sk), dtype=np.uint32))
+    _join(bj, oracle, torch_cuda, data, use_bloom=bloom, emit_key=True)
+
+
+def test_one_key(bj, oracle, torch_cuda):
+    """Every row of both sides has the same key: one bucket, and more pieces than the list holds."""
+    rk, sk = np.full(5000, 0xDEADBEEF, np.uint32), np.full(700, 0xDEADBEEF, np.uint32)
+    data = (rk, np.arange(5000, dtype=np.uint32), sk, np.arange(700, dtype=np.uint32))
+    assert _join(bj, oracle, torch_cuda, data).count == 5000 * 700
+
+
+@pytest.mark.parametrize("n_r,n_s,direct", [(MAX_BUILD, 4_000_000, True), (MAX_BUILD + 1, 4_000_000, False),
+                                            (5_000_000, MAX_BUILD, True)])
+@pytest.mark.parametrize("bloom", [0, 1])
+def test_limits(bj, oracle, torch_cuda, n_r, n_s, direct, bloom):
+    n0 = bj.kernel_launches()
+    _join(bj, oracle, torch_cuda, bj.gen_host(9, n_r, n_s, 0.2), launches=0, use_bloom=bloom)
+    assert (bj.kernel_launches() - n0 == 1) == direct
+
+
+def test_misaligned_overflow_and_reuse(bj, oracle, torch_cuda):
+    data = bj.gen_host(3, 70_001, 90_003, 0.4)
+    exp = oracle.pairs(*data)
+    with bj.Join(use_bloom=1) as j:
+        for cap in (len(exp[0]), 1000, 0, len(exp[0])):
+            st, r, s, _ = run_device(bj, torch_cuda, *data, cap=cap, handle=j, offset=(1, 2, 3, 1))
+            assert st.count == len(exp[0]) and st.overflow == (cap < len(exp[0])) and len(r) == cap
+            if cap == len(exp[0]):
+                assert_same_pairs(oracle, r, s, *exp)
+            else:
+                assert set(zip(r.tolist(), s.tolist())) <= set(zip(exp[0].tolist(), exp[1].tolist()))
