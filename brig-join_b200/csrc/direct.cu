@@ -81,14 +81,6 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
 }
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-// The whole 16-byte units of [lo, hi).
-__device__ __forceinline__ void prefetch_l2_bulk(const void* lo, const void* hi) {
-    const uintptr_t a = ((uintptr_t)lo + 15) & ~(uintptr_t)15, b = (uintptr_t)hi & ~(uintptr_t)15;
-    if (b > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(b - a)) : "memory");
-}
 __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -176,31 +168,10 @@ struct Side {
         if constexpr (kPacked) return __ldcg(&kv[i].y);
         else return __ldcs(v + i);
     }
-    __device__ __forceinline__ void prefetch_value(uint32_t i) const {
-        if constexpr (!kPacked) prefetch_l2(v + i);  // a packed value came with its key
-    }
-    __device__ __forceinline__ void prefetch_keys(uint64_t a, uint64_t b) const {
-        if constexpr (kPacked) prefetch_l2_bulk(kv + a, kv + b);
-        else prefetch_l2_bulk(k + a, k + b);
-    }
-    __device__ __forceinline__ void prefetch_values(uint64_t a, uint64_t b) const {
-        if constexpr (!kPacked) prefetch_l2_bulk(v + a, v + b);
-    }
 };
 template <bool kPacked>
 __device__ __forceinline__ Side<kPacked> side_of(const DirectJoin& d, int rel) {
     return Side<kPacked>{d.key[rel], d.val[rel], d.cmp};
-}
-
-// Brings rows [row, row + kStep) of a side's keys (and, kValues, its values) into L2, one bulk prefetch
-// per array by one lane. An SM's loads return through L1 in order: a row load that waits for DRAM holds
-// up the random reads behind it, which L2 could answer. So rows are in L2 before they are loaded.
-template <bool kValues, class S>
-__device__ __forceinline__ void prefetch_step(const S& side, uint64_t row, uint32_t n, int lane) {
-    if (row >= n) return;
-    const uint64_t end = min((uint64_t)n, row + kStep);
-    if (lane == 0) side.prefetch_keys(row, end);
-    if (kValues && lane == 1) side.prefetch_values(row, end);
 }
 
 // Loads this lane's rows row0 + 32 * u + lane below n (zeros at or past it).
@@ -216,16 +187,13 @@ __device__ __forceinline__ void load_step(const S& side, uint64_t row0, uint32_t
 // The rows of a phase are dealt to the warps of the grid in steps of kStep, round robin. Streams this
 // warp's steps of a side, the next step's rows loaded before f runs: f(row, keys)
 // with key u of this lane at row `row` + 32 * u.
-template <bool kValues, class S, class F>
+template <class S, class F>
 __device__ __forceinline__ void stream(const Ctx& c, const S& side, uint32_t row0, uint32_t n, F&& f) {
     const uint64_t stride = (uint64_t)c.nw * kStep;
     uint32_t t[kU];
-    prefetch_step<kValues>(side, row0 + stride, n, c.lane);
-    prefetch_step<kValues>(side, row0 + 2 * stride, n, c.lane);
     load_step(side, row0, n, c.lane, t);
     for (uint64_t r = row0; r < n; r += stride) {
         uint32_t nt[kU];
-        prefetch_step<kValues>(side, r + 3 * stride, n, c.lane);
         load_step(side, r + stride, n, c.lane, nt);
         f((uint32_t)r + c.lane, t);
 #pragma unroll
@@ -485,7 +453,7 @@ __device__ __noinline__ void phase_filter_build(Ctx& c, const uint2* pat) {
         const uint32_t nb = c.s.role.nb;
         uint2* dir = d.dir;
         uint32_t* rank = d.rank;
-        stream<false>(c, side_of<false>(d, 0), row0, n, [&](uint32_t row, const uint32_t (&t)[kU]) {
+        stream(c, side_of<false>(d, 0), row0, n, [&](uint32_t row, const uint32_t (&t)[kU]) {
             uint32_t q[kU];
 #pragma unroll
             for (int u = 0; u < kU; ++u) {
@@ -497,7 +465,7 @@ __device__ __noinline__ void phase_filter_build(Ctx& c, const uint2* pat) {
                 if (row + 32u * u < n) rank[row + 32u * u] = q[u];
         });
     } else {
-        stream<false>(c, side_of<false>(d, 0), row0, n, [&](uint32_t row, const uint32_t (&t)[kU]) {
+        stream(c, side_of<false>(d, 0), row0, n, [&](uint32_t row, const uint32_t (&t)[kU]) {
 #pragma unroll
             for (int u = 0; u < kU; ++u) insert(t[u], row + 32u * u < n);
         });
@@ -528,9 +496,6 @@ __device__ __noinline__ void phase_filter_probe(Ctx& c, const uint2* pat) {
                 w[u] = __ldcg(reinterpret_cast<const uint2*>(bloom + bloom_slot(m, f, seg).widx));
         }
     };
-    prefetch_step<false>(side, row0 + stride, n, c.lane);
-    prefetch_step<false>(side, row0 + 2 * stride, n, c.lane);
-    prefetch_step<false>(side, row0 + 3 * stride, n, c.lane);
     load_step(side, row0, n, c.lane, t);
     words((uint64_t)row0 + c.lane);
     load_step(side, row0 + stride, n, c.lane, nt);
@@ -539,17 +504,12 @@ __device__ __noinline__ void phase_filter_probe(Ctx& c, const uint2* pat) {
         for (int u = 0; u < kU; ++u) {
             const bool pass = bloom_pass(w[u], slot_masks<K>(pat, bloom_slot(mix32(t[u]), 0u, seg)));
             const uint32_t b = __ballot_sync(0xffffffffu, pass);
-            if (pass) {
-                const uint32_t i = (uint32_t)r + 32u * u + c.lane;
-                q[qn + __popc(b & lanemask_lt())] = make_uint2(t[u], i);
-                side.prefetch_value(i);
-            }
+            if (pass) q[qn + __popc(b & lanemask_lt())] = make_uint2(t[u], (uint32_t)r + 32u * u + c.lane);
             qn += __popc(b);
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) t[u] = nt[u];
         words(r + stride + c.lane);  // on their way while survivors are written
-        prefetch_step<false>(side, r + 4 * stride, n, c.lane);
         load_step(side, r + 2 * stride, n, c.lane, nt);
         if (qn >= 128) {
             qn -= 128;
@@ -583,7 +543,7 @@ __device__ __forceinline__ void count_run(const Ctx& c, const DirectJoin& d, con
     uint2* dir = d.dir;
     uint32_t* rank = d.rank;
     const uint32_t nb = r.nb;
-    stream<false>(c, side_of<kPacked>(d, rel), row0, n, [&](uint32_t row, const uint32_t (&t)[kU]) {
+    stream(c, side_of<kPacked>(d, rel), row0, n, [&](uint32_t row, const uint32_t (&t)[kU]) {
         uint32_t q[kU];
         bool on[kU];
 #pragma unroll
@@ -606,7 +566,7 @@ __device__ __forceinline__ void place_run(const Ctx& c, const DirectJoin& d, con
     uint2* table = d.table;
     const uint32_t nb = r.nb, cap = d.build_cap;
     const Side<kPacked> side = side_of<kPacked>(d, rel);
-    stream<true>(c, side, row0, n, [&](uint32_t row, const uint32_t (&t)[kU]) {
+    stream(c, side, row0, n, [&](uint32_t row, const uint32_t (&t)[kU]) {
         uint32_t pos[kU], v[kU];
         bool on[kU];
 #pragma unroll
@@ -781,9 +741,6 @@ __device__ __noinline__ uint32_t probe_run(const Ctx& c, const DirectJoin& d, co
         }
     };
     int qn = 0;
-    prefetch_step<false>(side, row0 + stride, n, c.lane);
-    prefetch_step<false>(side, row0 + 2 * stride, n, c.lane);
-    prefetch_step<false>(side, row0 + 3 * stride, n, c.lane);
     load_step(side, row0, n, c.lane, t);
     entries((uint64_t)row0 + c.lane);
     load_step(side, row0 + stride, n, c.lane, nt);
@@ -797,14 +754,12 @@ __device__ __noinline__ uint32_t probe_run(const Ctx& c, const DirectJoin& d, co
                 ws.q.key[at] = t[u];
                 ws.q.row[at] = (uint32_t)r0 + 32u * u + c.lane;
                 ws.q.entry[at] = (e[u].x << 8) | (e[u].y & kCntMask);
-                side.prefetch_value((uint32_t)r0 + 32u * u + c.lane);
             }
             qn += __popc(b);
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) t[u] = nt[u];
         entries(r0 + stride + c.lane);
-        prefetch_step<false>(side, r0 + 4 * stride, n, c.lane);
         load_step(side, r0 + 2 * stride, n, c.lane, nt);
         while (qn >= 32) {  // the queue's end first: its order does not matter
             const int k = min(qn, 64);
