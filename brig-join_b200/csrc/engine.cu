@@ -271,10 +271,7 @@ void layout_for(const brig_join_config& cfg, const JoinPlan* plans, int nj, int 
     sh.tcount = L.take(((size_t)sh.total_domains + 1) * 4);
     sh.toff = L.take(((size_t)sh.total_domains + 1) * 8);
     sh.tasks = L.take((size_t)sh.task_cap * sizeof(Task));
-    sh.scan_tmp_len = std::max({scan_tmp_words(std::max(sh.hist_len[0], sh.hist_len[1])),
-                                scan_tmp_words(sh.total_domains + 1), scan_tmp_words(sh.total_segs + 1),
-                                scan_tmp_words(std::max(sh.h2_len[0], sh.h2_len[1]))});
-    sh.scan_tmp = L.take((size_t)sh.scan_tmp_len * 8);
+    sh.scan_tmp = L.take((size_t)kScanMaxCtas * 8);
     sh.gwords = L.take(kGWords * 8);
     sh.counters = L.take((size_t)nj * kCntWords * 8);
     sh.meta_bytes = (size_t)nj * sizeof(JoinDesc) + 5 * ((size_t)nj + 1) * 8;
@@ -621,7 +618,6 @@ void fill_pipeline(const brig_join_config& cfg, const JoinPlan* plans, const Joi
     a.tasks = reinterpret_cast<Task*>(ws + sh.tasks);
     a.task_cap = sh.task_cap;
     a.scan_tmp = reinterpret_cast<int64_t*>(ws + sh.scan_tmp);
-    a.scan_tmp_len = sh.scan_tmp_len;
     a.gwords = reinterpret_cast<unsigned long long*>(ws + sh.gwords);
     a.max_p1 = sh.max_p1;
     a.max_p2 = sh.max_p2;

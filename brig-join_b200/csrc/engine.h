@@ -77,7 +77,6 @@ struct Shape {
     size_t seg_ns = 0, seg_off = 0, hist2 = 0, hist2_scan = 0, slice_cnt2 = 0;
     int64_t h2_len[2] = {0, 0};
     int64_t l2_slice_cap[2] = {0, 0};
-    int64_t scan_tmp_len = 0;
     size_t meta_bytes = 0;      // descriptor image: nj JoinDesc + 5 prefix arrays of nj+1 int64
     size_t total = 0;           // workspace bytes
     int max_p1 = 1, max_p2 = 1, max_seg_words = 0, bloom_smem_words = 0;

@@ -4,10 +4,10 @@
 //   gpu_prefix_init + gpu_run_hist_for_both (src/kernel_functions.cu:22-90,141-159) -> k_l1_hist
 //   queryAndCompactKernelPartitioned (src/bloom.cu:725-773), fused into S's histogram pass
 //                                                                            -> k_l1_hist (Bloom)
-//   gpu_make_simple_prefix (src/kernel_functions.cu:461-492)          -> k_scan_* (device-wide)
+//   gpu_make_simple_prefix (src/kernel_functions.cu:461-492)          -> k_scan_one, k_scan_grid
 //   gpu_make_sorted_table_for_both (src/kernel_functions.cu:95-133)    -> k_l1_scatter
 //   gpu_run_hist_second_pass + gpu_build_table_second_pass_kv (src/kernel_functions.cu:163-281)
-//                                     -> k_l2_plan + k_l2_hist + k_l2_scatter + k_l2_bounds
+//                                     -> k_l2_hist + k_l2_scatter + k_l2_bounds
 //   queryAndCompactKernelPartitioned, alternatively as S's level-2 pass      -> k_l2_bloom
 //   insertKernelPartitioned (src/bloom.cu:698-722)                     -> k_bloom_build
 //   gpu_probe_with_second_pass / gpu_fused_probe_transfer local part
@@ -882,9 +882,11 @@ k_l1_scatter(const JoinDesc* __restrict__ J, int nj, int rel, const int64_t* __r
     if constexpr (kBulk) bulk_wait_all();  // the bulk stores have written the output before the kernel ends
 }
 
-// Level-1 partition starts of every join with P2 == 1, or the level-2 input ranges otherwise:
-// b1[p] = start of partition p in l1, b1[P1] = relation total. One thread per entry.
-__global__ void k_bounds_l1(const JoinDesc* __restrict__ J, int nj, int rel, const int64_t* __restrict__ scan) {
+// Level-1 partition starts of every join: b1[p] = start of partition p in l1, b1[P1] = relation total. For
+// joins with a second level also the level-2 slices of each partition (at least one, so every partition
+// owns a histogram region). One thread per entry.
+__global__ void k_bounds_l1(const JoinDesc* __restrict__ J, int nj, int rel, const int64_t* __restrict__ scan,
+                            const int64_t* __restrict__ seg_prefix, uint32_t* __restrict__ seg_ns) {
     for (int j = blockIdx.y; j < nj; j += gridDim.y) {
         const JoinDesc& d = J[j];
         const RelPlan& R = d.rel[rel];
@@ -892,14 +894,21 @@ __global__ void k_bounds_l1(const JoinDesc* __restrict__ J, int nj, int rel, con
         const int64_t* S = scan + R.hist_base;
         int64_t* b1 = R.b1;
         const int64_t s0 = S[0];
-        for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p <= P1; p += gridDim.x * blockDim.x)
-            b1[p] = S[(int64_t)p * R.nslices] - s0;
+        for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p <= P1; p += gridDim.x * blockDim.x) {
+            const int64_t start = S[(int64_t)p * R.nslices] - s0;
+            b1[p] = start;
+            if (d.pf.P2 > 1 && p < P1) {
+                const int64_t len = S[(int64_t)(p + 1) * R.nslices] - s0 - start;
+                seg_ns[seg_prefix[j] + p] = (uint32_t)max_i64(1, (len + R.l2_slice - 1) / R.l2_slice);
+            }
+        }
     }
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) seg_ns[seg_prefix[nj]] = 0;  // the scan's last entry
 }
 
 // ---- Level 2 ------------------------------------------------------------------------------------
 // Every level-1 partition p is cut into slices of R.l2_slice tuples, planned on the device
-// (k_l2_plan + a scan of the slice counts). Slices are handed to CTAs in (join, p, slice) order,
+// (k_bounds_l1 + a scan of the slice counts). Slices are handed to CTAs in (join, p, slice) order,
 // so the CTAs running at any moment work on a few adjacent partitions: their output runs and, for
 // a level-2 Bloom probe, their filter segments stay in L2. Per join the level-2 histogram is laid
 // out [p][q][slice]; one exclusive scan of it gives every (p, q, slice) its output run, the same
@@ -932,20 +941,6 @@ __device__ __forceinline__ L2Slice l2_decode(const int64_t* __restrict__ seg_pre
     x.sl = t - seg_off[lo];
     x.local_off = seg_off[lo] - seg_off[seg_prefix[x.j]];
     return x;
-}
-
-// Slices per level-1 partition (at least one, so every partition owns a histogram region).
-__global__ void k_l2_plan(const JoinDesc* __restrict__ J, int nj, int rel, const int64_t* __restrict__ seg_prefix,
-                          uint32_t* __restrict__ seg_ns) {
-    const int64_t total = seg_prefix[nj];
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g <= total; g += (int64_t)gridDim.x * blockDim.x) {
-        if (g == total) { seg_ns[g] = 0; continue; }
-        const int j = find_owner(seg_prefix, nj, g);
-        const RelPlan& R = J[j].rel[rel];
-        const int64_t p = g - seg_prefix[j];
-        const int64_t len = R.b1[p + 1] - R.b1[p];
-        seg_ns[g] = (uint32_t)max_i64(1, (len + R.l2_slice - 1) / R.l2_slice);
-    }
 }
 
 // Level-2 histogram of one slice: counts by level-2 id. Handles every slice except those of S in
@@ -1831,60 +1826,85 @@ __global__ void k_publish_counts(const JoinDesc* __restrict__ J, int nj, const u
     }
 }
 
-// ---- device-wide exclusive scan (uint32 -> int64), three kernels -------------------------------
+// ---- device-wide exclusive scan (uint32 -> int64), one kernel -----------------------------------
+// A run scans seven small arrays (513 to 1.5M counts), each between two kernels that need all of it, so a
+// scan costs its launches and little else. Up to kScanOne counts one CTA walks them; above that a
+// cooperative grid of at most one CTA per SM sums its share, waits for the others and writes its share.
+// With three launches per scan instead (sums, their scan, the rest) and the level-2 plan in a kernel of
+// its own, a 16M x 16M join took 765 us against 722 us, a 4M x 16M join 909 against 856 us.
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kThreads * kScanItems;
+constexpr int64_t kScanOne = 2 * kScanTile;
 
-__global__ void __launch_bounds__(kThreads) k_scan_reduce(const uint32_t* __restrict__ in, int64_t n,
-                                                          int64_t* __restrict__ sums) {
-    __shared__ int64_t tmp[kThreads / 32];
-    const int64_t t0 = (int64_t)blockIdx.x * kScanTile;
-    int64_t s = 0;
-    for (int k = 0; k < kScanItems; ++k) {
-        const int64_t i = t0 + (int64_t)k * kThreads + threadIdx.x;
-        if (i < n) s += in[i];
-    }
-    int64_t total;
-    block_scan_excl_i64(s, tmp, &total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kThreads) k_scan_sums(int64_t* __restrict__ sums, int64_t nblk,
-                                                        int64_t* __restrict__ grand) {
-    __shared__ int64_t tmp[kThreads / 32];
-    int64_t carry = 0;
-    for (int64_t c0 = 0; c0 < nblk; c0 += kThreads) {
-        const int64_t i = c0 + threadIdx.x;
-        const int64_t v = i < nblk ? sums[i] : 0;
+// Exclusive scan of tiles [t0, t1) of `in`, starting from `carry`; returns the sum with it.
+__device__ int64_t scan_tiles(const uint32_t* __restrict__ in, int64_t n, int64_t t0, int64_t t1, int64_t carry,
+                              int64_t* __restrict__ out, int64_t* tmp) {
+    for (int64_t t = t0; t < t1; ++t) {
+        const int64_t i0 = t * kScanTile + (int64_t)threadIdx.x * kScanItems;
+        uint32_t v[kScanItems];
+        int64_t s = 0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = i0 + k < n ? in[i0 + k] : 0u;
+            s += v[k];
+        }
         int64_t total;
-        const int64_t ex = block_scan_excl_i64(v, tmp, &total);
-        if (i < nblk) sums[i] = carry + ex;
+        int64_t run = block_scan_excl_i64(s, tmp, &total) + carry;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            if (i0 + k < n) out[i0 + k] = run;
+            run += v[k];
+        }
         carry += total;
     }
-    if (threadIdx.x == 0 && grand) *grand = carry;
+    return carry;
 }
 
-__global__ void __launch_bounds__(kThreads) k_scan_down(const uint32_t* __restrict__ in, int64_t n,
-                                                        const int64_t* __restrict__ sums,
-                                                        int64_t* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) k_scan_one(const uint32_t* __restrict__ in, int64_t n,
+                                                        int64_t* __restrict__ out, int64_t* __restrict__ grand) {
     __shared__ int64_t tmp[kThreads / 32];
-    const int64_t t0 = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
+    const int64_t total = scan_tiles(in, n, 0, (n + kScanTile - 1) / kScanTile, 0, out, tmp);
+    if (threadIdx.x == 0 && grand) *grand = total;
+}
+
+// arrivals: the run's count of CTAs that have passed a scan's first half, `want` of them after this scan's.
+// The wait is bounded like the other waits of the pipeline; a CTA that gives up counts an error and
+// leaves its share unwritten.
+__global__ void __launch_bounds__(kThreads) k_scan_grid(const uint32_t* __restrict__ in, int64_t n, int64_t* sums,
+                                                         int64_t* __restrict__ out, int64_t* __restrict__ grand,
+                                                         unsigned long long* arrivals, unsigned long long want,
+                                                         unsigned long long* errors) {
+    __shared__ int64_t tmp[kThreads / 32];
+    __shared__ int s_ok;
+    const int64_t tiles = (n + kScanTile - 1) / kScanTile;
+    const int64_t t0 = tiles * blockIdx.x / gridDim.x, t1 = tiles * (blockIdx.x + 1) / gridDim.x;
     int64_t s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const int64_t i = t0 + k;
-        v[k] = i < n ? in[i] : 0u;
-        s += v[k];
-    }
+    for (int64_t i = t0 * kScanTile + threadIdx.x; i < t1 * kScanTile && i < n; i += kThreads) s += in[i];
     int64_t total;
-    int64_t run = block_scan_excl_i64(s, tmp, &total) + sums[blockIdx.x];
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-        const int64_t i = t0 + k;
-        if (i < n) out[i] = run;
-        run += v[k];
+    block_scan_excl_i64(s, tmp, &total);
+    if (threadIdx.x == 0) {
+        sums[blockIdx.x] = total;
+        __threadfence();
+        atomicAdd(arrivals, 1ull);
+        bool ok = false;
+        for (uint32_t it = 0; it < kDefaultPolls && !ok; ++it) {
+            unsigned long long v;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(arrivals) : "memory");
+            ok = v >= want;
+            if (!ok && it > 64) __nanosleep(100);
+        }
+        if (!ok) atomicAdd(errors, 1ull);
+        s_ok = ok ? 1 : 0;
+        __threadfence();
     }
+    __syncthreads();
+    if (!s_ok) return;  // block-uniform
+    int64_t before = 0;  // at most one CTA per SM: one sum per thread
+    if (threadIdx.x < blockIdx.x) before = __ldcg(sums + threadIdx.x);
+    int64_t carry;
+    block_scan_excl_i64(before, tmp, &carry);
+    const int64_t end = scan_tiles(in, n, t0, t1, carry, out, tmp);
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0 && grand) *grand = end;
 }
 
 // Resets the run's state words: the task queue, the error count (unless the run continues an earlier
@@ -1892,6 +1912,7 @@ __global__ void __launch_bounds__(kThreads) k_scan_down(const uint32_t* __restri
 __global__ void k_init_words(unsigned long long* g, int keep_errors, uint32_t polls) {
     g[kGQueue] = 0ull;
     if (!keep_errors) g[kGErrors] = 0ull;
+    g[kGScanArrivals] = 0ull;
     g[kGWaitPolls] = polls;
 }
 
@@ -1920,17 +1941,23 @@ const char* stage_name(int i) {
     return (i >= 0 && i < kNumStages) ? names[i] : nullptr;
 }
 
-int64_t scan_tmp_words(int64_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
-
-cudaError_t enqueue_scan(const uint32_t* in, int64_t* out, int64_t n, int64_t* tmp, int64_t* total,
-                         cudaStream_t st) {
+// Exclusive scan of n counts; writes the sum to *total (device pointer, may be null). `arrivals`: CTAs of
+// the run's scans so far (its device count is the state word kGScanArrivals).
+static cudaError_t enqueue_scan(const PipelineArgs& a, const uint32_t* in, int64_t* out, int64_t n, int64_t* total,
+                                unsigned long long& arrivals, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const int64_t nblk = (n + kScanTile - 1) / kScanTile;
-    k_scan_reduce<<<(unsigned)nblk, kThreads, 0, st>>>(in, n, tmp);
-    k_scan_sums<<<1, kThreads, 0, st>>>(tmp, nblk, total);
-    k_scan_down<<<(unsigned)nblk, kThreads, 0, st>>>(in, n, tmp, out);
-    note_launches(3);
-    return cudaGetLastError();
+    note_launches(1);
+    if (n <= kScanOne) {
+        k_scan_one<<<1, kThreads, 0, st>>>(in, n, out, total);
+        return cudaGetLastError();
+    }
+    const int64_t tiles = (n + kScanTile - 1) / kScanTile;
+    const int grid = (int)std::min<int64_t>({tiles, (int64_t)a.num_sms, kThreads, kScanMaxCtas});
+    arrivals += (unsigned long long)grid;
+    int64_t* sums = a.scan_tmp;
+    unsigned long long *word = a.gwords + kGScanArrivals, *errors = a.gwords + kGErrors;
+    void* args[] = {&in, &n, &sums, &out, &total, &word, &arrivals, &errors};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_scan_grid), dim3(grid), dim3(kThreads), args, 0, st);
 }
 
 size_t probe_smem_bytes(int table_cap, int emit_key) {
@@ -2037,6 +2064,7 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
     const int sms = a.num_sms;
 
     int launches = 0;
+    unsigned long long arrivals = 0;
     auto mark = [&](int i) {
         if (a.stage_events) cudaEventRecord(a.stage_events[i], st);
     };
@@ -2073,8 +2101,8 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
             });
         }
         mark(m0);
-        if ((err = enqueue_scan(a.hist + a.hist_begin[rel], a.hist_scan + a.hist_begin[rel],
-                                a.hist_len[rel], a.scan_tmp, nullptr, st)) != cudaSuccess)
+        if ((err = enqueue_scan(a, a.hist + a.hist_begin[rel], a.hist_scan + a.hist_begin[rel], a.hist_len[rel], nullptr,
+                                arrivals, st)) != cudaSuccess)
             return err;
         mark(m0 + 1);
         if (a.total_slices[rel] > 0) {
@@ -2099,15 +2127,12 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
         mark(m0 + 2);
         {
             dim3 grid((unsigned)((a.max_p1 + 1 + 255) / 256), (unsigned)std::min(a.nj, 65535));
-            k_bounds_l1<<<grid, 256, 0, st>>>(a.J, a.nj, rel, a.hist_scan);
+            k_bounds_l1<<<grid, 256, 0, st>>>(a.J, a.nj, rel, a.hist_scan, a.seg_prefix, a.seg_ns);
             ++launches;
         }
         if (a.total_segs > 0) {
-            const int pb = (int)std::min<int64_t>((a.total_segs + 1 + 255) / 256, (int64_t)sms * 8);
-            k_l2_plan<<<pb, 256, 0, st>>>(a.J, a.nj, rel, a.seg_prefix, a.seg_ns);
-            ++launches;
-            if ((err = enqueue_scan(a.seg_ns, a.seg_off, a.total_segs + 1, a.scan_tmp,
-                                    reinterpret_cast<int64_t*>(a.gwords + kGL2Slices + rel), st)) != cudaSuccess)
+            if ((err = enqueue_scan(a, a.seg_ns, a.seg_off, a.total_segs + 1,
+                                    reinterpret_cast<int64_t*>(a.gwords + kGL2Slices + rel), arrivals, st)) != cudaSuccess)
                 return err;
             uint32_t* h2 = a.hist2 + a.h2_begin[rel];
             if ((err = cudaMemsetAsync(h2, 0, (size_t)a.h2_len[rel] * 4, st)) != cudaSuccess) return err;
@@ -2130,7 +2155,7 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
                 });
             }
             mark(m0 + 3);
-            if ((err = enqueue_scan(h2, a.hist2_scan + a.h2_begin[rel], a.h2_len[rel], a.scan_tmp, nullptr, st)) !=
+            if ((err = enqueue_scan(a, h2, a.hist2_scan + a.h2_begin[rel], a.h2_len[rel], nullptr, arrivals, st)) !=
                 cudaSuccess)
                 return err;
             for_modes(a.modes, [&](auto mt) {
@@ -2165,8 +2190,8 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
         const int blocks = (int)std::min<int64_t>((n + kTaskWarps - 1) / kTaskWarps, (int64_t)sms * 16);
         k_tasks_count<<<blocks, kTaskWarps * 32, 0, st>>>(a.J, a.nj, a.dom_prefix, a.tcount);
         ++launches;
-        if ((err = enqueue_scan(a.tcount, a.toff, n, a.scan_tmp,
-                                reinterpret_cast<int64_t*>(a.gwords + kGTasks), st)) != cudaSuccess)
+        if ((err = enqueue_scan(a, a.tcount, a.toff, n, reinterpret_cast<int64_t*>(a.gwords + kGTasks), arrivals, st)) !=
+            cudaSuccess)
             return err;
         k_tasks_write<<<blocks, kTaskWarps * 32, 0, st>>>(a.J, a.nj, a.dom_prefix, a.toff, a.tasks, a.task_cap,
                                                           a.gwords);

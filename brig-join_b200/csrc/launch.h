@@ -30,8 +30,7 @@ struct PipelineArgs {
     int64_t* toff;                    // exclusive scan of tcount
     Task* tasks;                      // task list
     int64_t task_cap;
-    int64_t* scan_tmp;                // block sums for the device-wide scan
-    int64_t scan_tmp_len;
+    int64_t* scan_tmp;                // [kScanMaxCtas] block sums of the device-wide scan
     unsigned long long* gwords;       // [kGWords]
     int max_p1, max_p2;               // over the batch (shared-memory sizing)
     int max_seg_words;                // largest Bloom segment (words)
@@ -75,11 +74,7 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t stream);
 // Shared memory the probe kernel needs for a table of `table_cap` tuples.
 size_t probe_smem_bytes(int table_cap, int emit_key);
 
-// Device-wide exclusive scan of n uint32 counts into int64 offsets; writes the sum to *total
-// (device pointer, may be null). tmp must hold scan_tmp_words(n) int64.
-int64_t scan_tmp_words(int64_t n);
-cudaError_t enqueue_scan(const uint32_t* in, int64_t* out, int64_t n, int64_t* tmp,
-                         int64_t* total, cudaStream_t stream);
+constexpr int64_t kScanMaxCtas = 512;  // CTAs of a scan (one per SM): one block sum each
 
 // Input generator (gen.cu).
 cudaError_t enqueue_gen(uint64_t seed, int64_t n_r, int64_t n_s, double match_frac, double zipf_s,
