@@ -127,12 +127,13 @@ typedef struct brig_join_stats {
     int64_t written;             /* min(count, capacity) */
     int64_t s_survivors;         /* S tuples that passed the Bloom filter (= |S| when off)
                                     (BF candidate rate, src/hash_kernel.cu:1176-1179) */
-    int64_t tasks;               /* probe tasks executed */
+    int64_t tasks;               /* probe tasks executed (1: a small join that ran unpartitioned) */
     int64_t split_tasks;         /* tasks on the oversized-partition path (probe overflow blocks,
                                     src/kernel_functions.cu:356-358) */
     int32_t overflow;            /* 1 when count > capacity */
-    int32_t partition_size;      /* P1 used */
-    int32_t second_partition_size;/* P2 used */
+    int32_t partition_size;      /* P1 planned (of a small join that ran unpartitioned: P1 x P2 are the
+                                    filter's segments) */
+    int32_t second_partition_size;/* P2 planned */
     int32_t bloom_num_hashes;    /* k used (0 when off) */
     int64_t bloom_num_bits;      /* filter bits allocated (0 when off) */
     int64_t workspace_bytes;     /* device workspace held by the handle */
@@ -187,7 +188,8 @@ const char* brig_join_stage_name(int32_t i);
 /* Waits for the last run and writes the mean device time of each stage in milliseconds, over
  * the runs since the previous call (at most the last 64), into ms[BRIG_NUM_STAGES] (the
  * reference's per-stage timing table, src/hash_kernel.cu:1182-1358). Reading needs no
- * synchronisation between runs. A profiled handle launches its kernels directly instead of
+ * synchronisation between runs. A small join that runs as one kernel shows its time in the last stage.
+ * A profiled handle launches its kernels directly instead of
  * replaying a CUDA graph. BRIG_E_INVALID if the handle was created without profile_stages or
  * no run happened since the previous call. */
 int brig_join_stage_times(brig_join_t* h, double* ms, int32_t n);
