@@ -17,9 +17,11 @@
 //            one atomic on a cursor, so tiles need no order and no second barrier
 //   place    table[start + rank] = tuple
 //   probe    the other side streams through the directory and the table
-//   long     (only when a bucket exceeds kLockstep) the listed pieces of long buckets, spread over the
-//            grid: neighbouring rows of the streamed side often share their skew (Zipf ranks in row
-//            order), and a warp that walked its own rows' buckets held up the whole grid
+//   long     (only when a bucket exceeds kLockstep) the listed long buckets, spread over the grid in pieces:
+//            neighbouring rows of the streamed side often share their skew (Zipf ranks in row order), and a
+//            warp that walked its own rows' buckets held up the whole grid. Rows that the list has no room
+//            for are walked by warps that have done little or marked and listed in further rounds, two
+//            barriers each, so a round's work is bounded and even however many pairs the join has
 // A filtered join whose R is the build side (`fused`) builds R's table beside the filter and probes S's
 // survivors on the spot: four barriers instead of seven, and no survivors written.
 //
@@ -36,11 +38,15 @@ constexpr int kU = 4;                        // rows per lane and step
 constexpr uint32_t kStep = kU * 32;          // rows a warp takes per step
 constexpr int kWarps = kThreads / 32;
 constexpr int kLockstep = 8;                 // longest bucket the lanes walk in lock step; others are listed
-constexpr uint32_t kLongPiece = 256;         // most entries of a listed piece
+constexpr uint32_t kLongPiece = 256;         // entries of a listed bucket that are walked together
+constexpr uint32_t kLongPieces = 1 << 22;    // most pieces of a round (10 ms of walking)
+constexpr uint32_t kWalkAhead = 65536;       // entries a warp may walk itself beyond its share (1 ms)
+constexpr uint32_t kWalkHere = 64;           // longest bucket that a warp beyond it walks all the same
 constexpr int kStage = 128;                  // pairs staged per warp
 constexpr int kQueue = 160;                  // streamed rows queued per warp for the table: 31 and a step's
 constexpr int kPacked = 256;                 // survivors queued per warp: 127 and a step's
 constexpr int kSeen = 1024;                  // keys a CTA remembers while it builds a filter
+static_assert(32ull * (kDirectMaxBuild / kLongPiece + 1) <= kLongPieces, "a warp's buckets fit an empty list");
 static_assert(kQueue >= 31 + (int)kStep && kPacked >= 127 + (int)kStep, "a step's rows fit");
 constexpr uint32_t kBarrierPolls = 1u << 25; // bound of a grid barrier's wait (each poll 0.2 us or more)
 
@@ -71,8 +77,13 @@ enum DirectWord : int {
     kDBarrier = 8,    // arrivals of all barriers so far
     kDExit = 9,       // CTAs that have finished
     kDLong = 10,      // some bucket is long
-    kDLongCount = 11, // entries of the long list
+    kDWalked = 11,    // entries of long buckets walked by the warps that met them
+    // In turn by round, so that the next round's are reset while this round's are read:
+    kDLongCount = 12, // buckets (high half) and pieces asked of the long list
+    kDLongEnd = 14,   // complement of the count at which the list was full (0: it was not)
+    kDLeft = 16,      // rows are marked for a further round
 };
+static_assert(kDLeft + 2 <= kDirectWords, "state words");
 // Counters of a join that only this kernel uses.
 enum DirectCounter : int { kCntCursor = 6 };  // table space handed out
 
@@ -98,6 +109,10 @@ struct Role {
 struct WarpShared {
     uint2 pair[kStage];
     uint32_t pair_key[kStage];
+    // of long buckets that the warp meets once the list is full: entries walked, of those reported to the
+    // grid's count, and the most it may walk as of its last report
+    unsigned long long walked, reported, may_walk;
+    uint32_t list_full;
     union {
         struct {
             uint32_t key[kQueue], row[kQueue], entry[kQueue];  // entry: start << 8 | min(count, 255)
@@ -359,39 +374,56 @@ __device__ __noinline__ uint32_t long_length(const uint2* table, uint32_t start,
     return lo + 1 - start;
 }
 
-// Lists the buckets of the lanes with len > 0 in pieces for phase_long; walks them here when the list
-// is full. Returns the staging count.
-__device__ __noinline__ int list_long(const DirectArgs* a, uint32_t key, uint32_t val,
-                                      uint32_t start, uint32_t len, uint32_t bs, int lane, uint2* buf, uint32_t* keys,
-                                      int count) {
-    const uint32_t pieces = (len + kLongPiece - 1) / kLongPiece;
+// Lists the buckets of the lanes with len > 0 for phase_long; false when the list has no room for all of
+// them (an empty list has). One atomic takes list entries and piece numbers together, so the first piece
+// numbers of the entries ascend.
+__device__ __noinline__ bool list_long(const DirectArgs* a, int round, uint32_t key, uint32_t val, uint32_t start,
+                                       uint32_t len, int lane) {
+    const uint32_t pieces = (len + kLongPiece - 1) / kLongPiece, on = __ballot_sync(0xffffffffu, len > 0);
     uint32_t inc = pieces;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, inc, s);
         if (lane >= s) inc += y;
     }
-    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned long long add = ((unsigned long long)__popc(on) << 32) | __shfl_sync(0xffffffffu, inc, 31);
+    auto room = [&](unsigned long long to) { return (to >> 32) <= a->long_cap && (uint32_t)to <= kLongPieces; };
     unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(&a->gwords[kDLongCount], (unsigned long long)total);
+    int fits = 0;
+    if (lane == 0) {
+        unsigned long long* count = &a->gwords[kDLongCount + (round & 1)];
+        if (room(__ldcg(count))) {  // a full list's count stays: at most one addition a warp goes beyond it
+            base = atomicAdd(count, add);
+            fits = room(base + add);
+            if (!fits) atomicMax(&a->gwords[kDLongEnd + (round & 1)], ~base);
+        }
+    }
+    fits = __shfl_sync(0xffffffffu, fits, 0);
     base = __shfl_sync(0xffffffffu, base, 0);
-    const bool fits = base + total <= a->long_cap;
-    for (uint32_t p = 0; p < pieces; ++p) {
-        const unsigned long long at = base + inc - pieces + p;
-        if (at < a->long_cap)
-            a->longs[at] = DirectLong{key, val, start + p * kLongPiece, fits ? min(kLongPiece, len - p * kLongPiece) : 0u};
+    if (fits && len > 0) {
+        const uint32_t at = (uint32_t)(base >> 32) + __popc(on & lanemask_lt());
+        a->longs[at] = DirectLong{key, val, start, len};
+        a->first[at] = (uint32_t)base + inc - pieces;
     }
     __syncwarp();
-    return fits ? count : walk_spread(&a->join, key, val, start, len, bs, lane, buf, keys, count);
+    return fits;
 }
 
 // The bucket [start, + cnt) of each lane beyond its first three tuples (already compared; cnt 0: none).
-// Returns the staging count.
-__device__ __noinline__ int probe_rest(const DirectArgs* a, uint32_t key, uint32_t val,
-                                       uint32_t start, uint32_t cnt, uint32_t nb, uint32_t bs, int lane, uint2* buf,
-                                       uint32_t* keys, int count) {
-    const DirectJoin& d = a->join;
-    Stage st{buf, keys, count};
+// row: index of the lane's row in the streamed side. Returns the staging count.
+// Long buckets are listed. Once the list is full, a warp walks its buckets itself while it stays within
+// kWalkAhead entries of twice what the grid's warps have walked so on average; a warp that holds more of them,
+// as where hot rows lie side by side, marks them for the next round. Marking all of them instead cost 1M x 1M
+// rows of 100 copies a key 2.2 ms against 0.75 ms; walking all of them, 200 neighbours that match 100K tuples
+// each 269 ms against 0.5 ms.
+__device__ __noinline__ int probe_rest(const Ctx* c, uint32_t key, uint32_t val, uint32_t row, uint32_t start,
+                                       uint32_t cnt, int count) {
+    const DirectArgs& a = c->a;
+    const DirectJoin& d = a.join;
+    WarpShared& ws = c->s.w[c->wid];
+    const int lane = c->lane;
+    const uint32_t bs = c->s.role.bs, nb = c->s.role.nb;
+    Stage st{ws.pair, ws.pair_key, count};
     const bool small = cnt <= kLockstep;
     const uint32_t most = __reduce_max_sync(0xffffffffu, small ? cnt : 0u);
     for (uint32_t t = 3; t < most; ++t) {
@@ -400,14 +432,33 @@ __device__ __noinline__ int probe_rest(const DirectArgs* a, uint32_t key, uint32
         if (in) x = __ldcg(d.table + start + t);
         stage_pair(d, st, in && x.x == key, bs ? val : x.y, bs ? x.y : val, key, lane);
     }
-    if (__any_sync(0xffffffffu, !small)) {
-        uint32_t len = small ? 0u : cnt - 3;
-        if (cnt == kCntMask)
-            len = long_length(d.table, start, (uint32_t)__ldcg(&d.counters[kCntCursor]), fastrange32(mix32(key), nb), nb) - 3;
-        __syncwarp();
-        return list_long(a, key, val, start + 3, len, bs, lane, buf, keys, st.count);
+    if (!__any_sync(0xffffffffu, !small)) return st.count;
+    uint32_t len = small ? 0u : cnt - 3;
+    if (cnt == kCntMask)
+        len = long_length(d.table, start, (uint32_t)__ldcg(&d.counters[kCntCursor]), fastrange32(mix32(key), nb), nb) - 3;
+    __syncwarp();
+    if (!ws.list_full && list_long(&a, 0, key, val, start + 3, len, lane)) return st.count;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, len);
+    int here = 0;
+    if (lane == 0) {
+        ws.list_full = 1;
+        const unsigned long long walked = ws.walked + total;
+        if (walked > ws.may_walk || walked - ws.reported > kWalkAhead / 4) {
+            const unsigned long long all = atomicAdd(&a.gwords[kDWalked], ws.walked - ws.reported);
+            ws.reported = ws.walked;
+            ws.may_walk = kWalkAhead + 2 * (all / c->nw);
+        }
+        here = walked <= ws.may_walk;
+        if (here) ws.walked = walked;
     }
-    return st.count;
+    here = __shfl_sync(0xffffffffu, here, 0);
+    if (!here && len > kWalkHere) {
+        atomicOr(&a.left[row >> 5], 1u << (row & 31));
+        a.gwords[kDLeft] = 1ull;
+        len = 0;
+    }
+    __syncwarp();
+    return walk_spread(&d, key, val, start + 3, len, bs, lane, ws.pair, ws.pair_key, st.count);
 }
 
 // ---- phases ------------------------------------------------------------------------------------------
@@ -658,7 +709,7 @@ __device__ __noinline__ void phase_scan(Ctx& c) {
 // value and the bucket's first three tuples are read together, the rest of longer buckets in probe_rest.
 template <int kPer, bool kPacked>
 __device__ __forceinline__ void probe_queued(const Ctx& c, const DirectJoin& d, const Side<kPacked>& side, uint32_t bs,
-                                             uint32_t nb, const uint32_t* qkey, const uint32_t* qrow, const uint32_t* qent,
+                                             const uint32_t* qkey, const uint32_t* qrow, const uint32_t* qent,
                                              int n, Stage& st) {
     __syncwarp();
     uint32_t key[kPer], val[kPer], e[kPer];
@@ -690,8 +741,8 @@ __device__ __forceinline__ void probe_queued(const Ctx& c, const DirectJoin& d, 
 #pragma unroll
         for (int h = 0; h < kPer; ++h)
             if ((more >> h) & 1u)
-                st.count = probe_rest(&c.a, key[h], val[h], e[h] >> 8, e[h] & kCntMask, nb, bs, c.lane, st.buf, st.keys,
-                                      st.count);
+                st.count = probe_rest(&c, key[h], val[h], 32 * h + c.lane < n ? qrow[32 * h + c.lane] : 0u, e[h] >> 8,
+                                      e[h] & kCntMask, st.count);
     }
     __syncwarp();
 }
@@ -707,6 +758,11 @@ __device__ __noinline__ uint32_t probe_run(const Ctx& c, const DirectJoin& d, co
                                            uint32_t row0, uint32_t n, const uint2* pat) {
     WarpShared& ws = c.s.w[c.wid];
     Stage st{ws.pair, ws.pair_key, 0};
+    if (c.lane == 0) {
+        ws.walked = ws.reported = 0;
+        ws.may_walk = kWalkAhead;
+        ws.list_full = 0;
+    }
     const uint32_t nb = r.nb, bs = r.bs;
     const uint2* dir = d.dir;
     const Side<kPacked> side = side_of<kPacked>(d, rel);
@@ -764,10 +820,10 @@ __device__ __noinline__ uint32_t probe_run(const Ctx& c, const DirectJoin& d, co
         while (qn >= 32) {  // the queue's end first: its order does not matter
             const int k = min(qn, 64);
             qn -= k;
-            probe_queued<2>(c, d, side, bs, nb, ws.q.key + qn, ws.q.row + qn, ws.q.entry + qn, k, st);
+            probe_queued<2>(c, d, side, bs, ws.q.key + qn, ws.q.row + qn, ws.q.entry + qn, k, st);
         }
     }
-    if (qn > 0) probe_queued<1>(c, d, side, bs, nb, ws.q.key, ws.q.row, ws.q.entry, qn, st);
+    if (qn > 0) probe_queued<1>(c, d, side, bs, ws.q.key, ws.q.row, ws.q.entry, qn, st);
     if (st.count > 0) flush_pairs(d, st, c.lane);
     return passed;
 }
@@ -784,10 +840,8 @@ __device__ __noinline__ void phase_probe(Ctx& c, const uint2* pat) {
             p = __reduce_add_sync(0xffffffffu, p);
             if (c.lane == 0 && p)
                 atomicAdd(reinterpret_cast<unsigned long long*>(&d.counters[kCntSurvivors]), (unsigned long long)p);
-        } else if (r.bs) {
+        } else {  // S's survivors are the build side
             probe_run<false, false, M, K>(c, d, r, 0, row0, r.pn, pat);
-        } else {
-            probe_run<true, false, M, K>(c, d, r, 1, row0, r.pn, pat);
         }
     } else {
         probe_run<false, false, M, K>(c, d, r, r.bs ? 0 : 1, row0, r.pn, pat);
@@ -795,17 +849,82 @@ __device__ __noinline__ void phase_probe(Ctx& c, const uint2* pat) {
 }
 
 // The long list: each warp takes up to 32 pieces at a time.
-__device__ __noinline__ void phase_long(Ctx& c) {
+__device__ __noinline__ void phase_long(Ctx& c, int round) {
     const DirectJoin& d = c.a.join;
-    const uint32_t n = (uint32_t)min((unsigned long long)c.a.long_cap, __ldcg(&c.a.gwords[kDLongCount]));
-    const uint32_t per = min(32u, (n + c.nw - 1) / c.nw), bs = c.s.role.bs;
+    const unsigned long long full = __ldcg(&c.a.gwords[kDLongEnd + (round & 1)]);
+    const unsigned long long end = full ? ~full : __ldcg(&c.a.gwords[kDLongCount + (round & 1)]);
+    const uint32_t n = (uint32_t)(end >> 32), pieces = (uint32_t)end;
+    const uint32_t per = min(32u, (pieces + c.nw - 1) / c.nw), bs = c.s.role.bs;
+    const uint32_t* first = c.a.first;
     Stage st{c.s.w[c.wid].pair, c.s.w[c.wid].pair_key, 0};
-    for (uint32_t i0 = c.gw * per; i0 < n; i0 += c.nw * per) {
+    for (uint32_t g0 = c.gw * per; g0 < pieces; g0 += c.nw * per) {
+        // e0: the entry of piece g0, the last whose first piece is not beyond it
+        uint32_t e0 = 0;
+        if (pieces == n) {
+            e0 = g0;
+        } else {
+            for (uint32_t span = n; span > 1;) {
+                const uint32_t step = (span + 31) / 32, at = step * c.lane;
+                const uint32_t b = __ballot_sync(0xffffffffu, at < span && __ldcg(first + e0 + min(at, span - 1)) <= g0);
+                const uint32_t k = step * (31 - __clz(b));
+                e0 += k;
+                span = min(step, span - k);
+            }
+        }
+        // every entry has a piece, so those of the 32 pieces are among the next 32 entries
+        const uint32_t f = e0 + c.lane < n ? __ldcg(first + e0 + c.lane) : 0xffffffffu, g = g0 + c.lane;
+        int i = 0;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+            if (__shfl_sync(0xffffffffu, f, i + s) <= g) i += s;
+        const uint32_t fi = __shfl_sync(0xffffffffu, f, i);
         uint4 p = make_uint4(0u, 0u, 0u, 0u);  // key, value, start, length
-        if (c.lane < per && i0 + c.lane < n) p = __ldcg(reinterpret_cast<const uint4*>(c.a.longs + i0 + c.lane));
+        if (c.lane < per && g < pieces) {
+            p = __ldcg(reinterpret_cast<const uint4*>(c.a.longs + e0 + i));
+            const uint32_t k = (g - fi) * kLongPiece;
+            p.z += k;
+            p.w = min(kLongPiece, p.w - k);
+        }
+        __syncwarp();
         st.count = walk_spread(&d, p.x, p.y, p.z, p.w, bs, c.lane, st.buf, st.keys, st.count);
     }
     if (st.count > 0) flush_pairs(d, st, c.lane);
+}
+
+// Lists the marked rows, 32 neighbours at a time, until the list has no room; those that it takes are
+// unmarked. The first 32 that a round lists always fit, so every round makes progress.
+__device__ __noinline__ void phase_relist(Ctx& c, int round) {
+    const DirectArgs& a = c.a;
+    const DirectJoin& d = a.join;
+    const Role r = c.s.role;
+    const Side<false> side = side_of<false>(d, r.bs ? 0 : 1);  // the streamed side is never packed
+    const uint32_t words = (r.pn + 31) / 32, end = (uint32_t)__ldcg(&d.counters[kCntCursor]);
+    for (uint32_t w0 = c.gw * 32; w0 < words; w0 += c.nw * 32) {
+        const uint32_t mine = w0 + c.lane < words ? __ldcg(a.left + w0 + c.lane) : 0u;
+        for (uint32_t todo = __ballot_sync(0xffffffffu, mine != 0); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t bits = __shfl_sync(0xffffffffu, mine, src);
+            const uint32_t row = (w0 + src) * 32 + c.lane;
+            uint32_t key = 0, val = 0, start = 0, len = 0;
+            if ((bits >> c.lane) & 1u) {
+                key = side.load(row);
+                val = side.value(row);
+                const uint32_t b = fastrange32(mix32(key), r.nb);
+                const uint2 e = __ldcg(d.dir + b);
+                start = e.x;
+                len = e.y & kCntMask;
+                if (len == kCntMask) len = long_length(d.table, start, end, b, r.nb);
+                start += 3;
+                len -= 3;
+            }
+            __syncwarp();
+            if (!list_long(&a, round, key, val, start, len, c.lane)) {
+                if (c.lane == 0) a.gwords[kDLeft + (round & 1)] = 1ull;
+                return;  // what is still marked waits for the next round
+            }
+            if (c.lane == 0) a.left[w0 + src] = 0u;
+        }
+    }
 }
 
 // Returns false when a barrier ran out.
@@ -836,12 +955,19 @@ __device__ bool run_join(Ctx& c, const uint2* pat) {
     phase_scan(c);
     if (!grid_barrier(c)) return false;
     const bool longs = __ldcg(&a.gwords[kDLong]) != 0;
+    if (longs) clear16(a.left, ((size_t)c.s.role.pn + 127) / 128 * 16);
     phase_build<kFilter, true>(c);
     if (!grid_barrier(c)) return false;
     phase_probe<M, K, kFilter>(c, pat);
-    if (longs) {
+    for (int round = 0; longs; ++round) {
         if (!grid_barrier(c)) return false;
-        phase_long(c);
+        const bool left = __ldcg(&a.gwords[kDLeft + (round & 1)]) != 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0)  // the next round's words, last read a round ago
+            for (int w : {kDLongCount, kDLongEnd, kDLeft}) a.gwords[w + (~round & 1)] = 0ull;
+        phase_long(c, round);
+        if (!left) break;
+        if (!grid_barrier(c)) return false;
+        phase_relist(c, round + 1);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (!kFilter) d.counters[kCntSurvivors] = d.n[1];
@@ -930,9 +1056,13 @@ void direct_layout(const JoinPlan& p, int ctas, DirectShape& sh) {
     sh.table = take((size_t)build * 8);
     sh.rank = take((size_t)build * 4);
     if (p.bloom && !sh.fused) sh.cmp = take((size_t)p.ns * 8);
-    // one streamed row per bucket above kLockstep, and the pieces of longer ones
-    sh.long_cap = (uint32_t)std::min<int64_t>(build / kLockstep + build / kLongPiece + 64, 1 << 22);
+    // One streamed row per bucket above kLockstep. A round over a full list costs two barriers and a look at
+    // the marks (10-20 us), so small build sides get up to 32768.
+    const int64_t stream = std::max(p.nr, p.ns);
+    sh.long_cap = (uint32_t)std::max(build / kLockstep + 64, std::min<int64_t>(stream / 4, 32768));
     sh.longs = take((size_t)sh.long_cap * sizeof(DirectLong));
+    sh.first = take((size_t)sh.long_cap * 4);
+    sh.left = take((size_t)(stream + 127) / 128 * 16);
     sh.total = off + 256;
     // Every resident CTA, fewer while the longer side gives each warp less than one step.
     const int64_t want = (std::max(p.nr, p.ns) + kStep * kWarps - 1) / (kStep * kWarps);
@@ -968,6 +1098,8 @@ void direct_fill(const JoinPlan& p, const JoinIO& io, const DirectShape& sh, cha
     a.gwords = reinterpret_cast<unsigned long long*>(ws + sh.gwords);
     a.longs = reinterpret_cast<DirectLong*>(ws + sh.longs);
     a.long_cap = sh.long_cap;
+    a.first = reinterpret_cast<uint32_t*>(ws + sh.first);
+    a.left = reinterpret_cast<uint32_t*>(ws + sh.left);
     a.pat_k = p.bloom && p.k != kBloomFastK ? p.k : 0;
 }
 

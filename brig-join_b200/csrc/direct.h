@@ -30,7 +30,7 @@ struct DirectJoin {
     uint32_t build_cap;       // most build tuples
 };
 
-// A piece [start, start + len) of a long bucket and the streamed tuple that it is compared with.
+// A long bucket [start, start + len) and the streamed tuple that it is compared with.
 struct DirectLong {
     uint32_t key, val, start, len;
 };
@@ -41,10 +41,12 @@ struct DirectArgs {
     unsigned long long* gwords; // [kDirectWords], zero at launch
     DirectLong* longs;          // [long_cap]
     uint32_t long_cap;
+    uint32_t* first;            // [long_cap] first piece number of each
+    uint32_t* left;             // a bit per streamed row: listed in a later round
     int32_t pat_k;              // k of the pattern table (0: none)
 };
 
-constexpr int kDirectWords = 16;
+constexpr int kDirectWords = 18;
 constexpr uint32_t kDirTile = 4096;          // directory entries per scan tile
 // Limits of the direct path. Engine time in us, partitioned / direct, 10% matches unless noted (|R| x |S|
 // in millions; "f": filter of 10 bits per key): 0.1 x 0.1 155 / 45, 0.3 x 1.2 f 219 / 65, 1 x 16 456 / 235,
@@ -58,7 +60,7 @@ constexpr int64_t kDirectMaxFilter = 56ll << 20; // filter bytes (random accesse
 
 // Workspace of one join (byte offsets).
 struct DirectShape {
-    size_t counters = 0, gwords = 0, bloom = 0, cmp = 0, dir = 0, rank = 0, table = 0, longs = 0, total = 0;
+    size_t counters = 0, gwords = 0, bloom = 0, cmp = 0, dir = 0, rank = 0, table = 0, longs = 0, first = 0, left = 0, total = 0;
     uint32_t dir_cap = 0, build_cap = 0, long_cap = 0;
     int32_t fused = 0;
     int grid = 1;

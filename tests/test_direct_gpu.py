@@ -59,6 +59,47 @@ def test_one_key(bj, oracle, torch_cuda):
     assert _join(bj, oracle, torch_cuda, data).count == 5000 * 700
 
 
+@pytest.mark.parametrize("copies,rows,n_r,n_s,bloom", [
+    (100_000, 200, 0, 500_000, 0), (100_000, 200, 0, 500_000, 1),  # few rows of long buckets: 400 pieces each
+    (300, 60_000, 0, 140_000, 0),           # more rows than the list holds (32768), walked where they are met
+    (5000, 3000, 0, 3000, 0),               # more rows than it holds of more entries than a warp may walk: rounds
+    (2100, 34_000, 0, 140_000, 1),          # rounds behind the filter
+    (2100, 34_000, 3_200_000, 20_000, 1),   # S's survivors build, rounds over R's rows
+])
+def test_hot_key_on_both_sides(bj, oracle, torch_cuda, copies, rows, n_r, n_s, bloom):
+    """A key with many copies on the build side whose streamed rows lie side by side, as in a sorted relation.
+    Exact pairs, and no slower than a small multiple of the partitioned join (a warp that walked its own
+    rows' buckets while the others waited took over a hundred times as long)."""
+    t = torch_cuda
+    if n_r > n_s:
+        copies, rows = rows, copies  # of the streamed R and of S
+    rk = t.arange(2, 2 * max(n_r, copies) + 2, 2, dtype=t.int32, device="cuda")
+    sk = t.arange(1, 2 * n_s + 1, 2, dtype=t.int32, device="cuda")
+    rk[len(rk) // 3 if n_r > copies else 0:][:copies] = 0
+    sk[n_s // 3 if n_s > rows else 0:][:rows] = 0
+    r0, s0 = int((rk == 0).nonzero()[0]), int((sk == 0).nonzero()[0])
+    rv, sv = (t.arange(len(k), dtype=t.int32, device="cuda") for k in (rk, sk))
+    out = [t.empty(copies * rows, dtype=t.int32, device="cuda") for _ in range(2)]
+    ms = []
+    for cfg in (dict(), dict(table_capacity=4096)):
+        with bj.Join(use_bloom=bloom, **cfg) as j:
+            took = []
+            for _ in range(4):
+                e = [t.cuda.Event(enable_timing=True) for _ in range(2)]
+                out[0].fill_(-1)
+                n0 = bj.kernel_launches()
+                e[0].record()
+                j.run(rk, rv, len(rk), sk, sv, len(sk), out[0], out[1], copies * rows)
+                e[1].record()
+                assert (bj.kernel_launches() - n0 == 1) == (not cfg)
+                assert j.stats().count == copies * rows
+                took.append(e[0].elapsed_time(e[1]))
+            pair = (out[0].long() - r0) * rows + (out[1] - s0)
+            assert t.equal(pair.sort().values, t.arange(copies * rows, device="cuda"))
+        ms.append(min(took[1:]))
+    assert ms[0] < 4 * ms[1] + 1.0, ms
+
+
 @pytest.mark.parametrize("n_r,n_s,direct", [(MAX_BUILD, 4_000_000, True), (MAX_BUILD + 1, 4_000_000, False),
                                             (5_000_000, MAX_BUILD, True)])
 @pytest.mark.parametrize("bloom", [0, 1])
