@@ -106,34 +106,6 @@ __device__ __forceinline__ uint32_t block_scan_excl(uint32_t* a, int n, uint32_t
     return block_scan_excl_n<kThreads>(a, n, tmp);
 }
 
-// Same for int64 values (one value per thread), returns the exclusive prefix of this thread.
-__device__ int64_t block_scan_excl_i64(int64_t v, int64_t* tmp /* kThreads/32 */, int64_t* total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    constexpr int kWarps = kThreads / 32;
-    int64_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) tmp[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-        int64_t w = lane < kWarps ? tmp[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int64_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < kWarps) tmp[lane] = w;
-    }
-    __syncthreads();
-    int64_t excl = x - v + (wid > 0 ? tmp[wid - 1] : 0);
-    *total = tmp[kWarps - 1];
-    __syncthreads();
-    return excl;
-}
-
 __device__ __forceinline__ const uint2* final_buf(const JoinDesc& d, int rel) {
     return d.pf.P2 > 1 ? d.rel[rel].l2 : d.rel[rel].l1;
 }
@@ -214,6 +186,11 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, unsign
     if (threadIdx.x == 0) atomicAdd(err, 1ull);
     for (uint32_t it = 0; it < kDefaultPolls; ++it)
         if (mbar_try_wait(bar, parity)) return;
+}
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
 }
 __device__ __forceinline__ uint32_t wait_polls(const unsigned long long* gwords) {
     return (uint32_t)gwords[kGWaitPolls];
@@ -1835,86 +1812,7 @@ __global__ void k_publish_counts(const JoinDesc* __restrict__ J, int nj, const u
     }
 }
 
-// ---- device-wide exclusive scan (uint32 -> int64), one kernel -----------------------------------
-// A run scans seven small arrays (513 to 1.5M counts), each between two kernels that need all of it, so a
-// scan costs its launches and little else. Up to kScanOne counts one CTA walks them; above that a
-// cooperative grid of at most one CTA per SM sums its share, waits for the others and writes its share.
-// With three launches per scan instead (sums, their scan, the rest) and the level-2 plan in a kernel of
-// its own, a 16M x 16M join took 765 us against 722 us, a 4M x 16M join 909 against 856 us.
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kThreads * kScanItems;
-constexpr int64_t kScanOne = 2 * kScanTile;
-
-// Exclusive scan of tiles [t0, t1) of `in`, starting from `carry`; returns the sum with it.
-__device__ int64_t scan_tiles(const uint32_t* __restrict__ in, int64_t n, int64_t t0, int64_t t1, int64_t carry,
-                              int64_t* __restrict__ out, int64_t* tmp) {
-    for (int64_t t = t0; t < t1; ++t) {
-        const int64_t i0 = t * kScanTile + (int64_t)threadIdx.x * kScanItems;
-        uint32_t v[kScanItems];
-        int64_t s = 0;
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
-            v[k] = i0 + k < n ? in[i0 + k] : 0u;
-            s += v[k];
-        }
-        int64_t total;
-        int64_t run = block_scan_excl_i64(s, tmp, &total) + carry;
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
-            if (i0 + k < n) out[i0 + k] = run;
-            run += v[k];
-        }
-        carry += total;
-    }
-    return carry;
-}
-
-__global__ void __launch_bounds__(kThreads) k_scan_one(const uint32_t* __restrict__ in, int64_t n,
-                                                        int64_t* __restrict__ out, int64_t* __restrict__ grand) {
-    __shared__ int64_t tmp[kThreads / 32];
-    const int64_t total = scan_tiles(in, n, 0, (n + kScanTile - 1) / kScanTile, 0, out, tmp);
-    if (threadIdx.x == 0 && grand) *grand = total;
-}
-
-// arrivals: the run's count of CTAs that have passed a scan's first half, `want` of them after this scan's.
-// The wait is bounded like the other waits of the pipeline; a CTA that gives up counts an error and
-// leaves its share unwritten.
-__global__ void __launch_bounds__(kThreads) k_scan_grid(const uint32_t* __restrict__ in, int64_t n, int64_t* sums,
-                                                         int64_t* __restrict__ out, int64_t* __restrict__ grand,
-                                                         unsigned long long* arrivals, unsigned long long want,
-                                                         unsigned long long* errors) {
-    __shared__ int64_t tmp[kThreads / 32];
-    __shared__ int s_ok;
-    const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-    const int64_t t0 = tiles * blockIdx.x / gridDim.x, t1 = tiles * (blockIdx.x + 1) / gridDim.x;
-    int64_t s = 0;
-    for (int64_t i = t0 * kScanTile + threadIdx.x; i < t1 * kScanTile && i < n; i += kThreads) s += in[i];
-    int64_t total;
-    block_scan_excl_i64(s, tmp, &total);
-    if (threadIdx.x == 0) {
-        sums[blockIdx.x] = total;
-        __threadfence();
-        atomicAdd(arrivals, 1ull);
-        bool ok = false;
-        for (uint32_t it = 0; it < kDefaultPolls && !ok; ++it) {
-            unsigned long long v;
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(arrivals) : "memory");
-            ok = v >= want;
-            if (!ok && it > 64) __nanosleep(100);
-        }
-        if (!ok) atomicAdd(errors, 1ull);
-        s_ok = ok ? 1 : 0;
-        __threadfence();
-    }
-    __syncthreads();
-    if (!s_ok) return;  // block-uniform
-    int64_t before = 0;  // at most one CTA per SM: one sum per thread
-    if (threadIdx.x < blockIdx.x) before = __ldcg(sums + threadIdx.x);
-    int64_t carry;
-    block_scan_excl_i64(before, tmp, &carry);
-    const int64_t end = scan_tiles(in, n, t0, t1, carry, out, tmp);
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0 && grand) *grand = end;
-}
+#include "scan.cuh"
 
 // Resets the run's state words: the task queue, the error count (unless the run continues an earlier
 // launch's count) and the bound of the waits.
@@ -1964,8 +1862,8 @@ static cudaError_t enqueue_scan(const PipelineArgs& a, const uint32_t* in, int64
     const int grid = (int)std::min<int64_t>({tiles, (int64_t)a.num_sms, kThreads, kScanMaxCtas});
     arrivals += (unsigned long long)grid;
     int64_t* sums = a.scan_tmp;
-    unsigned long long *word = a.gwords + kGScanArrivals, *errors = a.gwords + kGErrors;
-    void* args[] = {&in, &n, &sums, &out, &total, &word, &arrivals, &errors};
+    unsigned long long *word = a.gwords + kGScanArrivals, *polls = a.gwords + kGWaitPolls;
+    void* args[] = {&in, &n, &sums, &out, &total, &word, &arrivals, &polls};
     return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_scan_grid), dim3(grid), dim3(kThreads), args, 0, st);
 }
 

@@ -98,7 +98,9 @@ typedef struct brig_join_config {
                                        BRIG_E_INTERNAL and d_count reads -1) and waits once more, at
                                        most the default bound, for the copy in flight; 0 = 2^22 (the
                                        default), -1 = none, so every such wait reports the error at
-                                       once (a test of the error path; the results stay exact). The
+                                       once (a test of the error path; the results stay exact). A
+                                       scan's wait for its other CTAs has the same bound; when it runs
+                                       out the CTA computes what it waited for, which is no error. The
                                        reference's waits are unbounded (src/join_executor.cu:49) */
     int32_t partition_fill;         /* build-side tuples the planner aims for per finest partition, in
                                        percent of table_capacity (sets the level-2 fan-out; the

@@ -316,6 +316,21 @@ def test_bounded_waits_report_internal_error_and_stay_exact(bj, oracle, torch_cu
     assert st.count == n
 
 
+def test_scans_without_waits(bj, oracle, torch_cuda):
+    """wait_poll_limit = -1 at a size whose scans run on many CTAs (512 partitions x 592 slices): no CTA waits
+    for the others, each adds up what lies before its share, and the pairs are exact."""
+    rk, rv, sk, sv = bj.gen_host(78, 2_000_000, 3_000_000, 0.2)
+    exp_r, exp_s = oracle.pairs(rk, rv, sk, sv)
+    d = [torch_cuda.from_numpy(a.view(np.int32)).cuda() for a in (rk, rv, sk, sv)]
+    n = len(exp_r)
+    out = [torch_cuda.empty(n, dtype=torch_cuda.int32, device="cuda") for _ in range(2)]
+    with bj.Join(use_bloom=1, partition_size=512, second_partition_size=16, wait_poll_limit=-1) as j:
+        j.run(d[0], d[1], len(rk), d[2], d[3], len(sk), out[0], out[1], n)
+        with pytest.raises(bj.BrigError):  # the bulk copies' waits report their error
+            j.stats()
+    assert_same_pairs(oracle, *(o.cpu().numpy().view(np.uint32) for o in out), exp_r, exp_s)
+
+
 def test_gather_rate_helper(bj, torch_cuda):
     """brig_join_gather_rate (the benchmark's ceiling for the level-2 Bloom probe's filter reads)
     enqueues one kernel of the requested size and rejects tables that are not a power of two."""
