@@ -1026,14 +1026,23 @@ cudaError_t enqueue_direct(const DirectArgs& a, bool filter, int mode, int k, in
     return err;
 }
 
-bool direct_eligible(const brig_join_config& cfg, const JoinPlan& p) {
+bool direct_eligible(const brig_join_config& cfg, const JoinPlan& p, int64_t capacity) {
     // A caller that sets fan-outs, table sizes or wait bounds gets the partitioned join that has them.
     if (cfg.partition_size || cfg.second_partition_size || cfg.table_capacity || cfg.s_chunk || cfg.bloom_probe_level ||
         cfg.max_level1_bits || cfg.wait_poll_limit || cfg.partition_fill || cfg.slices_per_sm)
         return false;
-    const int64_t small = std::min(p.nr, p.ns);
-    return small >= 1 && small <= kDirectMaxBuild && std::max(p.nr, p.ns) <= kDirectMaxStream &&
-           (!p.bloom || p.bloom_bits / 8 <= kDirectMaxFilter);
+    const int64_t small = std::min(p.nr, p.ns), large = std::max(p.nr, p.ns);
+    if (small < 1 || small > kDirectMaxBuild || (p.bloom && p.bloom_bits / 8 > kDirectMaxFilter)) return false;
+    // room for the pairs of many rows: half of them, of a small table a quarter
+    const bool many = capacity >= (small < kDirectSmallTable ? large / 4 : large / 2), few_rows = small < kDirectFewRows;
+    int64_t limit = kDirectMaxStream;
+    if (p.ns > p.nr) {
+        if (many || few_rows || (p.bloom && small < kDirectFewFilterKeys)) limit = kDirectMidStream;
+        if (few_rows && (many || p.bloom)) limit = kDirectLowStream;
+    } else if (many && few_rows) {
+        limit = kDirectMidStream;
+    }
+    return large <= limit;
 }
 
 void direct_layout(const JoinPlan& p, int ctas, DirectShape& sh) {

@@ -285,7 +285,7 @@ int64_t Engine::workspace_needed(const brig_join_config& cfg, const std::vector<
     Shape sh;
     layout_for(cfg, plans.data(), (int)plans.size(), num_sms, jo.data(), sh);
     size_t total = sh.total;
-    if (plans.size() == 1 && direct_eligible(cfg, plans[0])) {
+    if (plans.size() == 1 && direct_eligible(cfg, plans[0], 0)) {
         DirectShape ds;
         direct_layout(plans[0], 2 * num_sms, ds);
         total = std::max(total, ds.total);
@@ -731,7 +731,7 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
     }
     std::vector<JoinPlan> plans = plan_batch(adapt_config(nj), nr.data(), ns.data(), nj, shared_l2_);
     // A direct join is one kernel whose descriptor is its argument, so a graph would save it nothing.
-    if (nj == 1 && direct_eligible(cfg_, plans[0])) {
+    if (nj == 1 && direct_eligible(cfg_, plans[0], joins[0].out.capacity)) {
         if (s_ready) cuda_check(cudaStreamWaitEvent(stream, s_ready, 0), "cudaStreamWaitEvent");
         run_direct(joins, plans, stream);
         return;

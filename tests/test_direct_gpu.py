@@ -109,6 +109,33 @@ def test_limits(bj, oracle, torch_cuda, n_r, n_s, direct, bloom):
     assert (bj.kernel_launches() - n0 == 1) == direct
 
 
+M = 1 << 20
+
+
+@pytest.mark.parametrize("n_r,n_s,many,bloom,direct", [
+    (M, 24 * M, 1, 0, True), (M, 24 * M + 1, 1, 0, False), (M, 48 * M, 0, 0, True), (M, 48 * M + 1, 0, 0, False),
+    (65_535, 24 * M + 1, 0, 1, False), (65_536, 24 * M + 1, 0, 1, True),  # a small filter
+    (8191, 24 * M + 1, 0, 0, False), (8191, 24 * M, 0, 0, True),          # few rows
+    (8191, 4 * M, 1, 1, True), (8191, 4 * M + 1, 1, 0, False), (8191, 4 * M + 1, 0, 1, False), (8192, 4 * M + 1, 1, 1, True),
+    (48 * M, M, 1, 0, True), (48 * M, 8192, 1, 0, True), (24 * M + 1, 8191, 1, 0, False), (24 * M + 1, 8191, 0, 0, True)])
+def test_limits_of_the_longer_side(bj, torch_cuda, n_r, n_s, many, bloom, direct):
+    """Where the partitioned join is the faster one it is taken: many pairs asked for, a filter or a smaller
+    side of few lines. Both give the same count."""
+    t = torch_cuda
+    d = [t.empty(n, dtype=t.int32, device="cuda") for n in (n_r, n_r, n_s, n_s)]
+    bj.gen_device(6, n_r, n_s, 0.05, 0.0, *d)
+    cap = max(n_r, n_s) // (4 if min(n_r, n_s) < 262_144 else 2) - (not many)
+    out = [t.empty(cap, dtype=t.int32, device="cuda") for _ in range(2)]
+    counts = []
+    for cfg in (dict(), dict(table_capacity=4096)):
+        with bj.Join(use_bloom=bloom, **cfg) as j:
+            n0 = bj.kernel_launches()
+            j.run(*d[:2], n_r, *d[2:], n_s, *out, cap)
+            assert (bj.kernel_launches() - n0 == 1) == (direct and not cfg)
+            counts.append(j.stats().count)
+    assert counts[0] == counts[1] == int(0.05 * n_s)
+
+
 def test_misaligned_overflow_and_reuse(bj, oracle, torch_cuda):
     data = bj.gen_host(3, 70_001, 90_003, 0.4)
     exp = oracle.pairs(*data)
