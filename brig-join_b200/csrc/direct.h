@@ -69,6 +69,11 @@ constexpr int64_t kDirectLowStream = 4 << 20;    // larger side where most rows 
 constexpr int64_t kDirectSmallTable = 256 << 10; // smaller side
 constexpr int64_t kDirectFewFilterKeys = 64 << 10;
 constexpr int64_t kDirectFewRows = 8 << 10;
+// Smaller side of a join whose S is still being copied from the host when it starts (whole call in us,
+// partitioned / direct): S the smaller 12 x 2 f 2369 / 2475, 20 x 3 f 3728 / 3955, 30 x 1 5097 / 4907;
+// R the smaller 3 x 6 f 1829 / 1893, 3 x 16 f 3820 / 3923, 2 x 7 1906 / 1876, 1 x 8 f 2045 / 1919.
+constexpr int64_t kDirectMaxLateR = 1 << 20;     // S, of a larger R
+constexpr int64_t kDirectMaxLateS = 2 << 20;     // R, of a larger S
 constexpr int64_t kDirectMaxFilter = 56ll << 20; // filter bytes (random accesses slow down above 64 MB)
 
 // Workspace of one join (byte offsets).

@@ -730,8 +730,12 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
         ns[j] = joins[j].ns;
     }
     std::vector<JoinPlan> plans = plan_batch(adapt_config(nj), nr.data(), ns.data(), nj, shared_l2_);
-    // A direct join is one kernel whose descriptor is its argument, so a graph would save it nothing.
-    if (nj == 1 && direct_eligible(cfg_, plans[0], joins[0].out.capacity)) {
+    bool direct = nj == 1 && direct_eligible(cfg_, plans[0], joins[0].out.capacity);
+    // While S is still being copied from the host, the partitioned join works on R; the direct join is one
+    // kernel that starts after the copy.
+    if (s_ready) direct = direct && std::min(nr[0], ns[0]) <= (nr[0] > ns[0] ? kDirectMaxLateR : kDirectMaxLateS);
+    // A direct join's descriptor is its kernel's argument, so a graph would save it nothing.
+    if (direct) {
         if (s_ready) cuda_check(cudaStreamWaitEvent(stream, s_ready, 0), "cudaStreamWaitEvent");
         run_direct(joins, plans, stream);
         return;

@@ -136,6 +136,20 @@ def test_limits_of_the_longer_side(bj, torch_cuda, n_r, n_s, many, bloom, direct
     assert counts[0] == counts[1] == int(0.05 * n_s)
 
 
+@pytest.mark.parametrize("n_r,n_s,direct", [(3_000_000, 3_000_000, True),  # one copy after the other, then the join
+                                            (7_500_000, 1 << 20, True), (7_500_000, (1 << 20) + 1, False),
+                                            (2 << 20, 7_500_000, True), ((2 << 20) + 1, 7_500_000, False)])
+def test_host_joins_overlap_the_copy_of_s(bj, oracle, n_r, n_s, direct):
+    data = bj.gen_host(12, n_r, n_s, 0.1)
+    exp = oracle.pairs(*data)
+    with bj.Join(use_bloom=1) as j:
+        n0 = bj.kernel_launches()
+        cnt, r, s = j.run_host(*data, capacity=len(exp[0]))
+        assert (bj.kernel_launches() - n0 == 1) == direct
+    assert cnt == len(exp[0])
+    assert_same_pairs(oracle, r, s, *exp)
+
+
 def test_misaligned_overflow_and_reuse(bj, oracle, torch_cuda):
     data = bj.gen_host(3, 70_001, 90_003, 0.4)
     exp = oracle.pairs(*data)
