@@ -314,7 +314,6 @@ enum GlobalWord : int {
     kGErrors = 2,          // device-side consistency failures
     kGL2Slices = 3,        // level-2 slices of R (word 3) and of S (word 4)
     kGWaitPolls = 5,       // polls after which a bounded wait gives up
-    kGScanArrivals = 6,    // CTAs that have passed the first half of a device-wide scan
     kGWords = 8
 };
 

@@ -617,7 +617,7 @@ void fill_pipeline(const brig_join_config& cfg, const JoinPlan* plans, const Joi
     a.toff = reinterpret_cast<int64_t*>(ws + sh.toff);
     a.tasks = reinterpret_cast<Task*>(ws + sh.tasks);
     a.task_cap = sh.task_cap;
-    a.scan_tmp = reinterpret_cast<int64_t*>(ws + sh.scan_tmp);
+    a.scan_tmp = reinterpret_cast<unsigned long long*>(ws + sh.scan_tmp);
     a.gwords = reinterpret_cast<unsigned long long*>(ws + sh.gwords);
     a.max_p1 = sh.max_p1;
     a.max_p2 = sh.max_p2;

@@ -1815,11 +1815,12 @@ __global__ void k_publish_counts(const JoinDesc* __restrict__ J, int nj, const u
 #include "scan.cuh"
 
 // Resets the run's state words: the task queue, the error count (unless the run continues an earlier
-// launch's count) and the bound of the waits.
-__global__ void k_init_words(unsigned long long* g, int keep_errors, uint32_t polls) {
+// launch's count), the bound of the waits and the sums of the scans. kScanMaxCtas threads.
+__global__ void k_init_words(unsigned long long* g, unsigned long long* scan_tmp, int keep_errors, uint32_t polls) {
+    scan_tmp[threadIdx.x] = 0ull;
+    if (threadIdx.x) return;
     g[kGQueue] = 0ull;
     if (!keep_errors) g[kGErrors] = 0ull;
-    g[kGScanArrivals] = 0ull;
     g[kGWaitPolls] = polls;
 }
 
@@ -1848,10 +1849,10 @@ const char* stage_name(int i) {
     return (i >= 0 && i < kNumStages) ? names[i] : nullptr;
 }
 
-// Exclusive scan of n counts; writes the sum to *total (device pointer, may be null). `arrivals`: CTAs of
-// the run's scans so far (its device count is the state word kGScanArrivals).
+// Exclusive scan of n counts; writes the sum to *total (device pointer, may be null). `tag`: the run's scans
+// on several CTAs so far.
 static cudaError_t enqueue_scan(const PipelineArgs& a, const uint32_t* in, int64_t* out, int64_t n, int64_t* total,
-                                unsigned long long& arrivals, cudaStream_t st) {
+                                unsigned long long& tag, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     note_launches(1);
     if (n <= kScanOne) {
@@ -1860,11 +1861,8 @@ static cudaError_t enqueue_scan(const PipelineArgs& a, const uint32_t* in, int64
     }
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
     const int grid = (int)std::min<int64_t>({tiles, (int64_t)a.num_sms, kThreads, kScanMaxCtas});
-    arrivals += (unsigned long long)grid;
-    int64_t* sums = a.scan_tmp;
-    unsigned long long *word = a.gwords + kGScanArrivals, *polls = a.gwords + kGWaitPolls;
-    void* args[] = {&in, &n, &sums, &out, &total, &word, &arrivals, &polls};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_scan_grid), dim3(grid), dim3(kThreads), args, 0, st);
+    k_scan_grid<<<grid, kThreads, 0, st>>>(in, n, a.scan_tmp, out, total, ++tag, a.gwords + kGWaitPolls);
+    return cudaGetLastError();
 }
 
 size_t probe_smem_bytes(int table_cap, int emit_key) {
@@ -1971,12 +1969,12 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
     const int sms = a.num_sms;
 
     int launches = 0;
-    unsigned long long arrivals = 0;
+    unsigned long long scans = 0;
     auto mark = [&](int i) {
         if (a.stage_events) cudaEventRecord(a.stage_events[i], st);
     };
     mark(0);
-    k_init_words<<<1, 1, 0, st>>>(a.gwords, a.keep_errors, a.wait_polls);
+    k_init_words<<<1, kScanMaxCtas, 0, st>>>(a.gwords, a.scan_tmp, a.keep_errors, a.wait_polls);
     ++launches;
 
     // ---- R, then S: level 1 and level 2 (the Bloom build sits between them) -----------------
@@ -2009,7 +2007,7 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
         }
         mark(m0);
         if ((err = enqueue_scan(a, a.hist + a.hist_begin[rel], a.hist_scan + a.hist_begin[rel], a.hist_len[rel], nullptr,
-                                arrivals, st)) != cudaSuccess)
+                                scans, st)) != cudaSuccess)
             return err;
         mark(m0 + 1);
         if (a.total_slices[rel] > 0) {
@@ -2039,7 +2037,7 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
         }
         if (a.total_segs > 0) {
             if ((err = enqueue_scan(a, a.seg_ns, a.seg_off, a.total_segs + 1,
-                                    reinterpret_cast<int64_t*>(a.gwords + kGL2Slices + rel), arrivals, st)) != cudaSuccess)
+                                    reinterpret_cast<int64_t*>(a.gwords + kGL2Slices + rel), scans, st)) != cudaSuccess)
                 return err;
             uint32_t* h2 = a.hist2 + a.h2_begin[rel];
             if ((err = cudaMemsetAsync(h2, 0, (size_t)a.h2_len[rel] * 4, st)) != cudaSuccess) return err;
@@ -2062,7 +2060,7 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
                 });
             }
             mark(m0 + 3);
-            if ((err = enqueue_scan(a, h2, a.hist2_scan + a.h2_begin[rel], a.h2_len[rel], nullptr, arrivals, st)) !=
+            if ((err = enqueue_scan(a, h2, a.hist2_scan + a.h2_begin[rel], a.h2_len[rel], nullptr, scans, st)) !=
                 cudaSuccess)
                 return err;
             for_modes(a.modes, [&](auto mt) {
@@ -2097,7 +2095,7 @@ cudaError_t enqueue_pipeline(const PipelineArgs& a, cudaStream_t st) {
         const int blocks = (int)std::min<int64_t>((n + kTaskWarps - 1) / kTaskWarps, (int64_t)sms * 16);
         k_tasks_count<<<blocks, kTaskWarps * 32, 0, st>>>(a.J, a.nj, a.dom_prefix, a.tcount);
         ++launches;
-        if ((err = enqueue_scan(a, a.tcount, a.toff, n, reinterpret_cast<int64_t*>(a.gwords + kGTasks), arrivals, st)) !=
+        if ((err = enqueue_scan(a, a.tcount, a.toff, n, reinterpret_cast<int64_t*>(a.gwords + kGTasks), scans, st)) !=
             cudaSuccess)
             return err;
         k_tasks_write<<<blocks, kTaskWarps * 32, 0, st>>>(a.J, a.nj, a.dom_prefix, a.toff, a.tasks, a.task_cap,

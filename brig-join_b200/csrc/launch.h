@@ -30,7 +30,7 @@ struct PipelineArgs {
     int64_t* toff;                    // exclusive scan of tcount
     Task* tasks;                      // task list
     int64_t task_cap;
-    int64_t* scan_tmp;                // [kScanMaxCtas] block sums of the device-wide scan
+    unsigned long long* scan_tmp;     // [kScanMaxCtas] block sums of the device-wide scans
     unsigned long long* gwords;       // [kGWords]
     int max_p1, max_p2;               // over the batch (shared-memory sizing)
     int max_seg_words;                // largest Bloom segment (words)

@@ -32,7 +32,7 @@ __device__ int64_t block_scan_excl_i64(int64_t v, int64_t* tmp /* kThreads/32 */
 
 // A run scans seven small arrays (513 to 1.5M counts), each between two kernels that need all of it, so a
 // scan costs its launches and little else. Up to kScanOne counts one CTA walks them; above that a
-// cooperative grid of at most one CTA per SM sums its share, waits for the others and writes its share.
+// grid of at most one CTA per SM sums its shares, waits for the sums before each and writes it.
 // With three launches per scan instead (sums, their scan, the rest) and the level-2 plan in a kernel of
 // its own, a 16M x 16M join took 765 us against 722 us, a 4M x 16M join 909 against 856 us.
 constexpr int kScanItems = 8;
@@ -70,39 +70,38 @@ __global__ void __launch_bounds__(kThreads) k_scan_one(const uint32_t* __restric
     if (threadIdx.x == 0 && grand) *grand = total;
 }
 
-// arrivals: the run's count of CTAs that have passed a scan's first half, `want` of them after this scan's.
-// The wait is bounded by *polls. A CTA whose wait runs out adds up the counts before its share itself (at
-// most a few MB from L2), so its share is written, and right, however long the others take.
-__global__ void __launch_bounds__(kThreads) k_scan_grid(const uint32_t* __restrict__ in, int64_t n, int64_t* sums,
-                                                         int64_t* __restrict__ out, int64_t* __restrict__ grand,
-                                                         unsigned long long* arrivals, unsigned long long want,
+// A share's sum is published in sums[blockIdx.x] under the scan's tag (a run's scans count up from 1, and the
+// run starts with cleared words), and thread t of a later CTA waits for share t. Every CTA publishes before it
+// waits, and for lower CTAs only, which the hardware starts first: the grid need not be resident together. The
+// wait is bounded by *polls; a CTA whose wait runs out adds up the counts before its share itself (at most a few
+// MB from L2), so its share is written, and right, however long the others take.
+constexpr int kScanTagShift = 48;  // sums are below 2^48
+__global__ void __launch_bounds__(kThreads) k_scan_grid(const uint32_t* __restrict__ in, int64_t n,
+                                                         unsigned long long* sums, int64_t* __restrict__ out,
+                                                         int64_t* __restrict__ grand, unsigned long long tag,
                                                          const unsigned long long* polls) {
     __shared__ int64_t tmp[kThreads / 32];
-    __shared__ int s_ok;
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
     const int64_t t0 = tiles * blockIdx.x / gridDim.x, t1 = tiles * (blockIdx.x + 1) / gridDim.x;
     int64_t s = 0;
     for (int64_t i = t0 * kScanTile + threadIdx.x; i < t1 * kScanTile && i < n; i += kThreads) s += in[i];
     int64_t total;
     block_scan_excl_i64(s, tmp, &total);
-    if (threadIdx.x == 0) {
-        sums[blockIdx.x] = total;
-        __threadfence();
-        atomicAdd(arrivals, 1ull);
+    if (threadIdx.x == 0) atomicExch(sums + blockIdx.x, (tag << kScanTagShift) | (unsigned long long)total);
+    bool ok = true;
+    int64_t before = 0;
+    if (threadIdx.x < blockIdx.x) {  // at most kThreads CTAs
         const uint32_t bound = (uint32_t)*polls;
-        bool ok = false;
+        ok = false;
         for (uint32_t it = 0; it < bound && !ok; ++it) {
-            ok = ld_acquire(arrivals) >= want;
+            const unsigned long long v = ld_acquire(sums + threadIdx.x);
+            ok = v >> kScanTagShift == tag;
+            before = (int64_t)(v & ((1ull << kScanTagShift) - 1));
             if (!ok && it > 64) __nanosleep(100);
         }
-        s_ok = ok ? 1 : 0;
-        __threadfence();
     }
-    __syncthreads();
-    int64_t before = 0;
-    if (s_ok) {  // at most one CTA per SM: one sum per thread
-        if (threadIdx.x < blockIdx.x) before = __ldcg(sums + threadIdx.x);
-    } else {
+    if (!__syncthreads_and(ok)) {
+        before = 0;
         for (int64_t i = threadIdx.x; i < t0 * kScanTile; i += kThreads) before += in[i];
     }
     int64_t carry;

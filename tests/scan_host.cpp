@@ -1,6 +1,6 @@
-// The scan kernels (scan.cuh) on the host: a CTA's threads are fibers and the CTAs run one after another, so
-// every CTA but the last waits for arrivals that do not come until its wait runs out. argv: n, grid, polls.
-// Prints "ok" when every offset and the total are right.
+// The scan kernels (scan.cuh) on the host: a CTA's threads are fibers and the CTAs run one after another: in
+// order, each with the sums that it waits for already there, or in reverse, where no wait succeeds.
+// argv: n, grid, polls, reverse. Prints "ok" when every offset and the total are right.
 #include <ucontext.h>
 #include <cstdint>
 #include <cstdio>
@@ -42,11 +42,18 @@ static int64_t __shfl_up_sync(unsigned, int64_t v, int d) {
     yield();
     return x;
 }
-static void __threadfence() {}
+static bool votes;
+static bool __syncthreads_and(bool v) {
+    __syncthreads();
+    votes = true;
+    __syncthreads();
+    votes = votes && v;
+    __syncthreads();
+    return votes;
+}
 static void __nanosleep(int) {}
-static int64_t __ldcg(const int64_t* p) { return *p; }
 static unsigned long long ld_acquire(const unsigned long long* p) { return *p; }
-static unsigned long long atomicAdd(unsigned long long* p, unsigned long long v) { return (*p += v) - v; }
+static void atomicExch(unsigned long long* p, unsigned long long v) { *p = v; }
 
 #include "scan.cuh"
 
@@ -79,14 +86,16 @@ int main(int, char** argv) {
     const int64_t n = atoll(argv[1]);
     gridDim.x = (unsigned)atoi(argv[2]);
     std::vector<uint32_t> in(n);
-    std::vector<int64_t> out(n, -1), sums(512, -1);
+    std::vector<int64_t> out(n, -1);
+    std::vector<unsigned long long> sums(512, (1ull << kScanTagShift) | 5);  // of an earlier scan
     int64_t total = -1, want = 0;
-    unsigned long long arrivals = 0, word = strtoull(argv[3], nullptr, 10);
+    const unsigned long long polls = strtoull(argv[3], nullptr, 10);
     for (int64_t i = 0; i < n; ++i) in[i] = (uint32_t)((i * 2654435761ull) >> 7) % 1000;
-    for (blockIdx.x = 0; blockIdx.x < gridDim.x; ++blockIdx.x) {
+    for (unsigned b = 0; b < gridDim.x; ++b) {
+        blockIdx.x = atoi(argv[4]) ? gridDim.x - 1 - b : b;
         body = [&] {
             if (gridDim.x == 1) k_scan_one(in.data(), n, out.data(), &total);
-            else k_scan_grid(in.data(), n, sums.data(), out.data(), &total, &arrivals, gridDim.x, &word);
+            else k_scan_grid(in.data(), n, sums.data(), out.data(), &total, 2, &polls);
         };
         run_cta();
     }

@@ -18,11 +18,12 @@ def scan(tmp_path_factory):
 
 @pytest.mark.parametrize("n", [1, 511, 4095, 4096, 4097, 8191, 8192])
 def test_one_cta(scan, n):
-    assert scan(n, 1, 0) == "ok"
+    assert scan(n, 1, 0, 0) == "ok"
 
 
 @pytest.mark.parametrize("n,grid", [(8193, 3), (12_288, 3), (12_289, 4), (50_001, 5), (200_000, 49)])
-@pytest.mark.parametrize("polls", [0, 100])
-def test_waits_that_run_out(scan, n, grid, polls):
-    """No CTA but the last sees the others arrive: each adds up what lies before its share itself."""
-    assert scan(n, grid, polls) == "ok"
+@pytest.mark.parametrize("polls,reverse", [(0, 0), (100, 0), (100, 1)])
+def test_many_ctas(scan, n, grid, polls, reverse):
+    """CTAs that find the sums before theirs, and CTAs whose wait for them runs out: these add up what lies
+    before their share themselves."""
+    assert scan(n, grid, polls, reverse) == "ok"
