@@ -696,7 +696,7 @@ void Engine::finish_run(const std::vector<JoinIO>& joins, const std::vector<Join
     nj_ = nj;
 }
 
-void Engine::run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream) {
+bool Engine::run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream) {
     const JoinPlan& p = plans[0];
     int& per_sm = direct_ctas_[!p.bloom ? 0 : 1 + 2 * (p.pf.mode != 0) + (p.k == kBloomFastK)];
     if (!per_sm) {
@@ -715,9 +715,15 @@ void Engine::run_direct(const std::vector<JoinIO>& joins, const std::vector<Join
     for (int i = 0; ev && i < kNumStages; ++i) cuda_check(cudaEventRecord(ev[i], stream), "cudaEventRecord");
     // the counters and the state words are adjacent
     cuda_check(cudaMemsetAsync(counters, 0, sh.gwords + kDirectWords * 8 - sh.counters, stream), "state reset");
-    cuda_check(enqueue_direct(a, p.bloom, p.pf.mode, p.k, sh.grid, stream), "direct join launch");
+    const cudaError_t err = enqueue_direct(a, p.bloom, p.pf.mode, p.k, sh.grid, stream);
+    if (err == cudaErrorCooperativeLaunchTooLarge) {  // a stream that owns fewer SMs than the device has
+        cudaGetLastError();
+        return false;
+    }
+    cuda_check(err, "direct join launch");
     if (ev) cuda_check(cudaEventRecord(ev[kNumStages], stream), "cudaEventRecord");
     finish_run(joins, plans, counters, a.gwords, stream);
+    return true;
 }
 
 void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use_graph, cudaEvent_t s_ready) {
@@ -737,8 +743,7 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
     // A direct join's descriptor is its kernel's argument, so a graph would save it nothing.
     if (direct) {
         if (s_ready) cuda_check(cudaStreamWaitEvent(stream, s_ready, 0), "cudaStreamWaitEvent");
-        run_direct(joins, plans, stream);
-        return;
+        if (run_direct(joins, plans, stream)) return;
     }
     std::vector<JoinOffs> jo(nj);
     Shape sh;

@@ -169,8 +169,9 @@ public:
                           cudaStream_t stream);
 
 private:
-    // The unpartitioned join (direct.cu) of a join that direct_eligible accepts.
-    void run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream);
+    // The unpartitioned join (direct.cu) of a join that direct_eligible accepts; false where the stream's SMs
+    // cannot hold its grid.
+    bool run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream);
     void finish_run(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, int64_t* counters,
                     unsigned long long* gwords, cudaStream_t stream);
     void ensure_workspace(size_t bytes, cudaStream_t stream);

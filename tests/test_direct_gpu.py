@@ -1,5 +1,9 @@
 """The unpartitioned join (one cooperative kernel) against the oracle and the partitioned join: step and
 tile remainders, both build sides, long buckets, the limits of the rule that chooses it."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -148,6 +152,34 @@ def test_host_joins_overlap_the_copy_of_s(bj, oracle, n_r, n_s, direct):
         assert (bj.kernel_launches() - n0 == 1) == direct
     assert cnt == len(exp[0])
     assert_same_pairs(oracle, r, s, *exp)
+
+
+SOME_SMS = """
+import torch, brig_join as bj
+t = torch.empty(1, device="cuda")
+green = torch.cuda.GreenContext.create(16, 0)
+green.set_context()
+st = torch.cuda.Stream()
+with torch.cuda.stream(st):
+    for n, cfg in ((1_000_000, {}), (1_000_000, dict(use_bloom=1)), (1 << 24, dict(use_bloom=1, use_cuda_graph=1))):
+        d = [torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(4)]
+        bj.gen_device(1, n, n, 0.1, 0.0, *d, stream=st.cuda_stream)
+        out = [torch.empty(n // 8, dtype=torch.int32, device="cuda") for _ in range(2)]
+        with bj.Join(**cfg) as j:
+            for _ in range(2):
+                j.run(*d[:2], n, *d[2:], n, *out, n // 8, stream=st.cuda_stream)
+                print(j.stats().count)
+green.pop_context()
+"""
+
+
+def test_stream_with_some_of_the_sms(torch_cuda):
+    """A stream of a context that owns 16 SMs cannot hold the cooperative grid: the join runs all the same."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.path.join(root, "brig-join_b200"))
+    r = subprocess.run([sys.executable, "-c", SOME_SMS], env=env, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert r.stdout.split() == ["100000"] * 4 + ["1677721"] * 2
 
 
 def test_misaligned_overflow_and_reuse(bj, oracle, torch_cuda):
