@@ -438,6 +438,16 @@ void Engine::ensure_host_io(int64_t nr, int64_t ns, int64_t cap, bool key) {
     }
 }
 
+// Waits for the work that a run has enqueued when the run fails before its end: nothing marks that work for the
+// handle's next run or its destruction, which free the workspace it uses.
+struct FailedRunWait {
+    cudaStream_t stream;
+    bool done = false;
+    ~FailedRunWait() {
+        if (!done) cudaStreamSynchronize(stream);
+    }
+};
+
 void Engine::run_host_chunked(const uint32_t* rk, const uint32_t* rv, int64_t nr, const uint32_t* sk,
                               const uint32_t* sv, int64_t ns, int chunks, int64_t cap, bool emit_key,
                               cudaStream_t st) {
@@ -479,6 +489,7 @@ void Engine::run_host_chunked(const uint32_t* rk, const uint32_t* rv, int64_t nr
                    "descriptor upload");
         cuda_check(enqueue_pipeline(a, st), "pipeline launch");
     };
+    FailedRunWait wait{st};
     // R: copied once, then its two passes and the Bloom build
     cuda_check(cudaMemcpyAsync(hio.rk, rk, (size_t)nr * 4, cudaMemcpyHostToDevice, st), "H2D R keys");
     cuda_check(cudaMemcpyAsync(hio.rv, rv, (size_t)nr * 4, cudaMemcpyHostToDevice, st), "H2D R vals");
@@ -513,6 +524,7 @@ void Engine::run_host_chunked(const uint32_t* rk, const uint32_t* rv, int64_t nr
     d_counters_ = counters;
     d_gwords_ = a.gwords;
     nj_ = 1;
+    wait.done = true;
 }
 
 void fill_pipeline(const brig_join_config& cfg, const JoinPlan* plans, const JoinIO* joins, int nj,
@@ -736,6 +748,7 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
         ns[j] = joins[j].ns;
     }
     std::vector<JoinPlan> plans = plan_batch(adapt_config(nj), nr.data(), ns.data(), nj, shared_l2_);
+    FailedRunWait wait{stream};
     bool direct = nj == 1 && direct_eligible(cfg_, plans[0], joins[0].out.capacity);
     // While S is still being copied from the host, the partitioned join works on R; the direct join is one
     // kernel that starts after the copy.
@@ -743,7 +756,7 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
     // A direct join's descriptor is its kernel's argument, so a graph would save it nothing.
     if (direct) {
         if (s_ready) cuda_check(cudaStreamWaitEvent(stream, s_ready, 0), "cudaStreamWaitEvent");
-        if (run_direct(joins, plans, stream)) return;
+        if ((wait.done = run_direct(joins, plans, stream))) return;
     }
     std::vector<JoinOffs> jo(nj);
     Shape sh;
@@ -834,6 +847,7 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
     if (use_graph) cuda_check(cudaEventRecord(stage_free_, stream), "cudaEventRecord");
     pipeline_loaded_ = true;
     finish_run(joins, plans, counters, a.gwords, stream);
+    wait.done = true;
 }
 
 // The adaptive filter's break-even: at |R| = 2^26, |S| = 2^30 and 10 bits/key the filtered join
