@@ -409,35 +409,39 @@ __device__ __noinline__ bool list_long(const DirectArgs* a, int round, uint32_t 
     return fits;
 }
 
-// The bucket [start, + cnt) of each lane beyond its first three tuples (already compared; cnt 0: none).
-// row: index of the lane's row in the streamed side. Returns the staging count.
+// The bucket [start, + cnt) of each lane beyond its first three tuples (already compared), in lock step; lanes with
+// more than kLockstep or at most three: none. Returns the staging count.
+__device__ __noinline__ int probe_rest(const DirectJoin* dp, uint32_t key, uint32_t val, uint32_t start, uint32_t cnt,
+                                       uint32_t bs, int lane, uint2* buf, uint32_t* keys, int count) {
+    const DirectJoin& d = *dp;
+    Stage st{buf, keys, count};
+    if (cnt > kLockstep) cnt = 0;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, cnt);
+    for (uint32_t t = 3; t < most; ++t) {
+        uint2 x = make_uint2(0u, 0u);
+        const bool in = t < cnt;
+        if (in) x = __ldcg(d.table + start + t);
+        stage_pair(d, st, in && x.x == key, bs ? val : x.y, bs ? x.y : val, key, lane);
+    }
+    return st.count;
+}
+
+// The same for the lanes with more than kLockstep tuples. row: index of the lane's row in the streamed side.
 // Long buckets are listed. Once the list is full, a warp walks its buckets itself while it stays within
 // kWalkAhead entries of twice what the grid's warps have walked so on average; a warp that holds more of them,
 // as where hot rows lie side by side, marks them for the next round. Marking all of them instead cost 1M x 1M
 // rows of 100 copies a key 2.2 ms against 0.75 ms; walking all of them, 200 neighbours that match 100K tuples
-// each 269 ms against 0.5 ms.
-__device__ __noinline__ int probe_rest(const Ctx* c, uint32_t key, uint32_t val, uint32_t row, uint32_t start,
-                                       uint32_t cnt, int count) {
-    const DirectArgs& a = c->a;
+// each 269 ms against 0.22 ms.
+__device__ __noinline__ int probe_long(const DirectArgs* ap, WarpShared* wp, uint32_t key, uint32_t val, uint32_t row,
+                                       uint32_t start, uint32_t cnt, uint32_t nb, uint32_t bs, int lane, int count) {
+    const DirectArgs& a = *ap;
     const DirectJoin& d = a.join;
-    WarpShared& ws = c->s.w[c->wid];
-    const int lane = c->lane;
-    const uint32_t bs = c->s.role.bs, nb = c->s.role.nb;
-    Stage st{ws.pair, ws.pair_key, count};
-    const bool small = cnt <= kLockstep;
-    const uint32_t most = __reduce_max_sync(0xffffffffu, small ? cnt : 0u);
-    for (uint32_t t = 3; t < most; ++t) {
-        uint2 x = make_uint2(0u, 0u);
-        const bool in = small && t < cnt;
-        if (in) x = __ldcg(d.table + start + t);
-        stage_pair(d, st, in && x.x == key, bs ? val : x.y, bs ? x.y : val, key, lane);
-    }
-    if (!__any_sync(0xffffffffu, !small)) return st.count;
-    uint32_t len = small ? 0u : cnt - 3;
+    WarpShared& ws = *wp;
+    uint32_t len = cnt > kLockstep ? cnt - 3 : 0u;
     if (cnt == kCntMask)
         len = long_length(d.table, start, (uint32_t)__ldcg(&d.counters[kCntCursor]), fastrange32(mix32(key), nb), nb) - 3;
     __syncwarp();
-    if (!ws.list_full && list_long(&a, 0, key, val, start + 3, len, lane)) return st.count;
+    if (!ws.list_full && list_long(&a, 0, key, val, start + 3, len, lane)) return count;
     const uint32_t total = __reduce_add_sync(0xffffffffu, len);
     int here = 0;
     if (lane == 0) {
@@ -446,7 +450,7 @@ __device__ __noinline__ int probe_rest(const Ctx* c, uint32_t key, uint32_t val,
         if (walked > ws.may_walk || walked - ws.reported > kWalkAhead / 4) {
             const unsigned long long all = atomicAdd(&a.gwords[kDWalked], ws.walked - ws.reported);
             ws.reported = ws.walked;
-            ws.may_walk = kWalkAhead + 2 * (all / c->nw);
+            ws.may_walk = kWalkAhead + 2 * (all / (gridDim.x * kWarps));
         }
         here = walked <= ws.may_walk;
         if (here) ws.walked = walked;
@@ -458,7 +462,7 @@ __device__ __noinline__ int probe_rest(const Ctx* c, uint32_t key, uint32_t val,
         len = 0;
     }
     __syncwarp();
-    return walk_spread(&d, key, val, start + 3, len, bs, lane, ws.pair, ws.pair_key, st.count);
+    return walk_spread(&d, key, val, start + 3, len, bs, lane, ws.pair, ws.pair_key, count);
 }
 
 // ---- phases ------------------------------------------------------------------------------------------
@@ -706,10 +710,11 @@ __device__ __noinline__ void phase_scan(Ctx& c) {
 }
 
 // Compares queued rows [0, n) of the streamed side with their buckets, up to kPer per lane: the row's
-// value and the bucket's first three tuples are read together, the rest of longer buckets in probe_rest.
+// value and the bucket's first three tuples are read together, the rest of longer buckets in probe_rest or
+// probe_long.
 template <int kPer, bool kPacked>
 __device__ __forceinline__ void probe_queued(const Ctx& c, const DirectJoin& d, const Side<kPacked>& side, uint32_t bs,
-                                             const uint32_t* qkey, const uint32_t* qrow, const uint32_t* qent,
+                                             uint32_t nb, const uint32_t* qkey, const uint32_t* qrow, const uint32_t* qent,
                                              int n, Stage& st) {
     __syncwarp();
     uint32_t key[kPer], val[kPer], e[kPer];
@@ -729,7 +734,8 @@ __device__ __forceinline__ void probe_queued(const Ctx& c, const DirectJoin& d, 
             x[h][k] = make_uint2(~key[h], 0u);
             if ((e[h] & kCntMask) > (uint32_t)k) x[h][k] = __ldcg(d.table + (e[h] >> 8) + k);
         }
-        more |= (e[h] & kCntMask) > 3 ? 1u << h : 0u;
+        const uint32_t cnt = e[h] & kCntMask;
+        more |= cnt > kLockstep ? 1u << (kPer + h) : cnt > 3 ? 1u << h : 0u;
     }
 #pragma unroll
     for (int h = 0; h < kPer; ++h)
@@ -739,10 +745,14 @@ __device__ __forceinline__ void probe_queued(const Ctx& c, const DirectJoin& d, 
     more = __reduce_or_sync(0xffffffffu, more);
     if (more) {
 #pragma unroll
-        for (int h = 0; h < kPer; ++h)
+        for (int h = 0; h < kPer; ++h) {
+            const uint32_t start = e[h] >> 8, cnt = e[h] & kCntMask;
             if ((more >> h) & 1u)
-                st.count = probe_rest(&c, key[h], val[h], 32 * h + c.lane < n ? qrow[32 * h + c.lane] : 0u, e[h] >> 8,
-                                      e[h] & kCntMask, st.count);
+                st.count = probe_rest(&d, key[h], val[h], start, cnt, bs, c.lane, st.buf, st.keys, st.count);
+            if ((more >> (kPer + h)) & 1u)
+                st.count = probe_long(&c.a, &c.s.w[c.wid], key[h], val[h], 32 * h + c.lane < n ? qrow[32 * h + c.lane] : 0u,
+                                      start, cnt, nb, bs, c.lane, st.count);
+        }
     }
     __syncwarp();
 }
@@ -820,10 +830,10 @@ __device__ __noinline__ uint32_t probe_run(const Ctx& c, const DirectJoin& d, co
         while (qn >= 32) {  // the queue's end first: its order does not matter
             const int k = min(qn, 64);
             qn -= k;
-            probe_queued<2>(c, d, side, bs, ws.q.key + qn, ws.q.row + qn, ws.q.entry + qn, k, st);
+            probe_queued<2>(c, d, side, bs, nb, ws.q.key + qn, ws.q.row + qn, ws.q.entry + qn, k, st);
         }
     }
-    if (qn > 0) probe_queued<1>(c, d, side, bs, ws.q.key, ws.q.row, ws.q.entry, qn, st);
+    if (qn > 0) probe_queued<1>(c, d, side, bs, nb, ws.q.key, ws.q.row, ws.q.entry, qn, st);
     if (st.count > 0) flush_pairs(d, st, c.lane);
     return passed;
 }
@@ -927,6 +937,22 @@ __device__ __noinline__ void phase_relist(Ctx& c, int round) {
     }
 }
 
+// Walks what the probe has listed, then lists and walks the marked rows until none is left. Returns false when
+// a barrier ran out.
+__device__ __noinline__ bool long_rounds(Ctx& c) {
+    const DirectArgs& a = c.a;
+    for (int round = 0;; ++round) {
+        if (!grid_barrier(c)) return false;
+        const bool left = __ldcg(&a.gwords[kDLeft + (round & 1)]) != 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0)  // the next round's words, last read a round ago
+            for (int w : {kDLongCount, kDLongEnd, kDLeft}) a.gwords[w + (~round & 1)] = 0ull;
+        phase_long(c, round);
+        if (!left) return true;
+        if (!grid_barrier(c)) return false;
+        phase_relist(c, round + 1);
+    }
+}
+
 // Returns false when a barrier ran out.
 template <int M, int K, bool kFilter>
 __device__ bool run_join(Ctx& c, const uint2* pat) {
@@ -959,16 +985,7 @@ __device__ bool run_join(Ctx& c, const uint2* pat) {
     phase_build<kFilter, true>(c);
     if (!grid_barrier(c)) return false;
     phase_probe<M, K, kFilter>(c, pat);
-    for (int round = 0; longs; ++round) {
-        if (!grid_barrier(c)) return false;
-        const bool left = __ldcg(&a.gwords[kDLeft + (round & 1)]) != 0;
-        if (blockIdx.x == 0 && threadIdx.x == 0)  // the next round's words, last read a round ago
-            for (int w : {kDLongCount, kDLongEnd, kDLeft}) a.gwords[w + (~round & 1)] = 0ull;
-        phase_long(c, round);
-        if (!left) break;
-        if (!grid_barrier(c)) return false;
-        phase_relist(c, round + 1);
-    }
+    if (longs && !long_rounds(c)) return false;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (!kFilter) d.counters[kCntSurvivors] = d.n[1];
         d.counters[kCntTasks] = 1;
