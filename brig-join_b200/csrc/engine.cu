@@ -708,6 +708,18 @@ void Engine::finish_run(const std::vector<JoinIO>& joins, const std::vector<Join
     nj_ = nj;
 }
 
+// Whether an output array shares memory with an input. The partitioned join has read all inputs before it writes
+// a pair, so pairs may replace inputs; the direct join reads them while it writes.
+static bool writes_inputs(const JoinIO& io) {
+    const uint32_t* in[] = {io.rk, io.rv, io.sk, io.sv};
+    for (const uint32_t* out : {io.out.r_val, io.out.s_val, io.out.key})
+        for (int i = 0; out && i < 4; ++i) {
+            const uintptr_t a = (uintptr_t)in[i], b = (uintptr_t)out;
+            if (a < b + (uintptr_t)io.out.capacity * 4 && b < a + (uintptr_t)(i < 2 ? io.nr : io.ns) * 4) return true;
+        }
+    return false;
+}
+
 bool Engine::run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream) {
     const JoinPlan& p = plans[0];
     int& per_sm = direct_ctas_[!p.bloom ? 0 : 1 + 2 * (p.pf.mode != 0) + (p.k == kBloomFastK)];
@@ -749,7 +761,7 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
     }
     std::vector<JoinPlan> plans = plan_batch(adapt_config(nj), nr.data(), ns.data(), nj, shared_l2_);
     FailedRunWait wait{stream};
-    bool direct = nj == 1 && direct_eligible(cfg_, plans[0], joins[0].out.capacity);
+    bool direct = nj == 1 && direct_eligible(cfg_, plans[0], joins[0].out.capacity) && !writes_inputs(joins[0]);
     // While S is still being copied from the host, the partitioned join works on R; the direct join is one
     // kernel that starts after the copy.
     if (s_ready) direct = direct && std::min(nr[0], ns[0]) <= (nr[0] > ns[0] ? kDirectMaxLateR : kDirectMaxLateS);

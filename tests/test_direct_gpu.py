@@ -154,6 +154,22 @@ def test_host_joins_overlap_the_copy_of_s(bj, oracle, n_r, n_s, direct):
     assert_same_pairs(oracle, r, s, *exp)
 
 
+@pytest.mark.parametrize("bloom", [0, 1])
+@pytest.mark.parametrize("over", [("rv", "sv"), ("rk", "sk"), ("sv", "rv")])
+def test_pairs_that_replace_the_inputs(bj, oracle, torch_cuda, over, bloom):
+    """Outputs in the memory of inputs (here 10 words into them), as the partitioned join allows."""
+    names = ("rk", "rv", "sk", "sv")
+    data = bj.gen_host(15, 300_000, 400_000, 0.5)
+    exp = oracle.pairs(*data)
+    n = len(exp[0])
+    d = {k: torch_cuda.from_numpy(a.view(np.int32)).cuda() for k, a in zip(names, data)}
+    out = [d[k][10:10 + n] for k in over]
+    with bj.Join(use_bloom=bloom) as j:
+        j.run(d["rk"], d["rv"], 300_000, d["sk"], d["sv"], 400_000, *out, n)
+        assert j.stats().count == n
+    assert_same_pairs(oracle, *(o.cpu().numpy().view(np.uint32) for o in out), *exp)
+
+
 SOME_SMS = """
 import torch, brig_join as bj
 t = torch.empty(1, device="cuda")
