@@ -279,13 +279,13 @@ void layout_for(const brig_join_config& cfg, const JoinPlan* plans, int nj, int 
     sh.total = L.off + 256;
 }
 
-int64_t Engine::workspace_needed(const brig_join_config& cfg, const std::vector<JoinPlan>& plans,
-                                 int num_sms) {
+int64_t Engine::workspace_needed(const brig_join_config& cfg, const std::vector<JoinPlan>& plans, int num_sms,
+                                 bool direct) {
     std::vector<JoinOffs> jo(plans.size());
     Shape sh;
     layout_for(cfg, plans.data(), (int)plans.size(), num_sms, jo.data(), sh);
     size_t total = sh.total;
-    if (plans.size() == 1 && direct_eligible(cfg, plans[0], 0)) {
+    if (direct && plans.size() == 1 && direct_eligible(cfg, plans[0], 0)) {
         DirectShape ds;
         direct_layout(plans[0], 2 * num_sms, ds);
         total = std::max(total, ds.total);
@@ -729,6 +729,7 @@ bool Engine::run_direct(const std::vector<JoinIO>& joins, const std::vector<Join
     }
     DirectShape sh;
     direct_layout(p, per_sm * num_sms_, sh);
+    if (reserved_only_ && sh.total > ws_bytes_) return false;
     if (have_run_) cuda_check(cudaStreamWaitEvent(stream, done_, 0), "cudaStreamWaitEvent");
     ensure_workspace(sh.total, stream);
     DirectArgs a;

@@ -132,9 +132,13 @@ public:
     // last kStageRing); returns the number of runs averaged (profile_stages only).
     int stage_times(double* ms, int n);
 
-    // Device workspace needed for these joins (bytes).
-    static int64_t workspace_needed(const brig_join_config& cfg, const std::vector<JoinPlan>& plans,
-                                    int num_sms);
+    // A direct join that needs more than the reserved workspace runs partitioned instead.
+    void set_reserved_only(bool on) { reserved_only_ = on; }
+
+    // Device workspace needed for these joins (bytes). direct: including that of a single join that may run
+    // unpartitioned, which can be the larger one.
+    static int64_t workspace_needed(const brig_join_config& cfg, const std::vector<JoinPlan>& plans, int num_sms,
+                                    bool direct = true);
 
     // Buffers owned by the engine for the host-array entry point.
     struct HostIOBufs {
@@ -170,7 +174,7 @@ public:
 
 private:
     // The unpartitioned join (direct.cu) of a join that direct_eligible accepts; false where the stream's SMs
-    // cannot hold its grid.
+    // cannot hold its grid or the reserved workspace its tables.
     bool run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream);
     void finish_run(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, int64_t* counters,
                     unsigned long long* gwords, cudaStream_t stream);
@@ -190,6 +194,7 @@ private:
     bool pipeline_loaded_ = false;   // the partitioned pipeline has run on this handle
     int direct_ctas_[5] = {};        // CTAs per SM of the unpartitioned join's kernels (0: not asked yet)
     bool shared_l2_ = false;
+    bool reserved_only_ = false;
     std::vector<JoinPlan> plans_;
     std::vector<int64_t> caps_;
     int64_t* d_counters_ = nullptr;  // [nj * kCntWords] of the last run

@@ -73,17 +73,17 @@ struct Server {
     static int64_t io_bytes(const brig_serve_request& r, int64_t cap) {
         return 8 * cap + (r.inputs_on_device ? 0 : 8 * (r.n_r + r.n_s));
     }
-    // io_bytes plus the workspace of the request joined alone (the admission bound).
+    // io_bytes plus the workspace of the request joined alone, partitioned (the admission bound).
     int64_t footprint(const brig_serve_request& r, int64_t cap) const {
-        return Engine::workspace_needed(jcfg, plan_batch(jcfg, &r.n_r, &r.n_s, 1, true), num_sms) + io_bytes(r, cap);
+        return Engine::workspace_needed(jcfg, plan_batch(jcfg, &r.n_r, &r.n_s, 1, true), num_sms, false) + io_bytes(r, cap);
     }
-    int64_t wave_workspace(const std::vector<Req*>& w) const {
+    int64_t wave_workspace(const std::vector<Req*>& w, bool direct) const {
         std::vector<int64_t> nr, ns;
         for (Req* q : w) {
             nr.push_back(q->in.n_r);
             ns.push_back(q->in.n_s);
         }
-        return Engine::workspace_needed(jcfg, plan_batch(jcfg, nr.data(), ns.data(), (int)w.size(), true), num_sms);
+        return Engine::workspace_needed(jcfg, plan_batch(jcfg, nr.data(), ns.data(), (int)w.size(), true), num_sms, direct);
     }
 
     // Request buffers are stream-ordered allocations on the slot's stream, so allocating and
@@ -215,8 +215,11 @@ struct Server {
                     auto is_large = [&](const Req* q) { return q->in.n_r + q->in.n_s > large_tuples; };
                     int64_t io = 0, ws_new = ws_have, tuples = 0;
                     auto fits = [&](const std::vector<Req*>& w, int64_t io2, int64_t& ws2) {
-                        ws2 = std::max(ws_have, wave_workspace(w));
-                        return used + io2 + (ws2 - ws_have) <= scfg.hbm_budget_bytes;
+                        for (bool direct : {true, false}) {  // unpartitioned only where the budget has room for it
+                            ws2 = std::max(ws_have, wave_workspace(w, direct));
+                            if (used + io2 + (ws2 - ws_have) <= scfg.hbm_budget_bytes) return true;
+                        }
+                        return false;
                     };
                     // slot 0: the oldest large request, alone
                     if (large_slot) {
@@ -392,6 +395,7 @@ int brig_serve_create(const brig_join_config* jcfg, const brig_serve_config* scf
                 brig::cuda_check(cudaEventCreateWithFlags(&sl.ev, cudaEventDisableTiming), "cudaEventCreate");
                 sl.eng = new brig::Engine(s->jcfg);
                 sl.eng->set_shared_l2(true);  // the slots' waves run side by side
+                sl.eng->set_reserved_only(true);
             }
         } catch (...) {
             for (auto& sl : s->slots) {

@@ -32,6 +32,21 @@ def test_every_request_matches_oracle(bj, oracle, torch_cuda):
     assert len(waves) > 1
 
 
+@pytest.mark.parametrize("room", [0, 64 << 20])
+def test_budget_of_the_partitioned_join_is_enough(bj, oracle, torch_cuda, room):
+    """A budget that holds a request's buffers and its partitioned workspace serves it, although the unpartitioned
+    join would need more."""
+    x = _req(bj, 5, 1_000_000, 1, 0.1)
+    er, es = oracle.pairs(*x)
+    need = bj.plan(1_000_000, 1_000_000, table_capacity=4096)[2]
+    assert need < bj.plan(1_000_000, 1_000_000)[2]
+    with bj.Server(hbm_budget_bytes=need + 8 * len(er) + 8 * 2_000_000 + room) as srv:
+        for _ in range(2):
+            res, a, b = srv.poll(srv.submit(*x, capacity=len(er)))
+            assert res.status == bj.BRIG_OK and res.count == len(er)
+            assert_same_pairs(oracle, a, b, er, es)
+
+
 def test_same_result_alone_and_in_mix(bj, oracle, torch_cuda):
     x = _req(bj, 77, 150_000, 4, 0.5)
     er, es = oracle.pairs(*x)
