@@ -28,6 +28,12 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
+// The last idle slot leaves a burst of small requests time to arrive: a wave goes there once no request has come
+// for kQuiet, or kGather after the launch before it. A lone request's join takes the host 8 us to launch, and
+// without this the first three of a burst took both slots and the rest waited for a whole wave (12 requests of
+// 65K x 262K submitted at once: median latency 0.74 ms against 0.57 ms when every launch took 0.1 ms).
+constexpr std::chrono::microseconds kQuiet(20), kGather(100);
+
 struct Req {
     int64_t ticket = 0;
     brig_serve_request in{};
@@ -66,6 +72,7 @@ struct Server {
     std::vector<Slot> slots;
     std::thread th;
     int next_wave = 0;
+    Clock::time_point last_launch;  // start of the latest wave's launch
     int device = 0;
     std::string fatal;
 
@@ -175,7 +182,7 @@ struct Server {
     void loop() {
         cudaSetDevice(device);
         for (;;) {
-            bool busy = false;
+            bool busy = false, gathering = false;
             for (auto& s : slots) {
                 if (s.phase == 0) continue;
                 busy = true;
@@ -190,6 +197,7 @@ struct Server {
                     fail_wave(s, BRIG_E_CUDA, cudaGetErrorString(q));
                 }
             }
+            size_t idle = std::count_if(slots.begin(), slots.end(), [](const Slot& s) { return s.phase == 0; });
             // admission. A request above large_mtuples tuples is large: large requests run one at a
             // time, each as a wave of its own, on slot 0, so two of them never share the GPU (which
             // would slow both and set the tail latency); the other slots batch and overlap the
@@ -242,7 +250,11 @@ struct Server {
                     // otherwise small requests in arrival order, passing any large one
                     const bool large_waiting =
                         std::any_of(pending.begin(), pending.end(), [&](const Req* q) { return is_large(q); });
-                    if (wave.empty() && !(large_slot && large_waiting)) {
+                    if (wave.empty() && idle == 1 && !pending.empty() && (int)pending.size() < scfg.max_wave) {
+                        const auto now = Clock::now();
+                        gathering = now - last_launch < kGather && now - pending.back()->t_submit < kQuiet;
+                    }
+                    if (wave.empty() && !gathering && !(large_slot && large_waiting)) {
                         for (auto it = pending.begin(); it != pending.end() && (int)wave.size() < scfg.max_wave;) {
                             Req* q = *it;
                             if (is_large(q)) {
@@ -301,6 +313,8 @@ struct Server {
                 }
                 s.wave = wave;
                 s.wave_id = next_wave++;
+                last_launch = Clock::now();
+                --idle;
                 try {
                     launch(s);
                 } catch (const Error& e) {
@@ -310,11 +324,13 @@ struct Server {
             }
             std::unique_lock<std::mutex> lk(mu);
             if (stop && pending.empty()) {
-                bool idle = true;
-                for (auto& s : slots) idle = idle && s.phase == 0;
-                if (idle) return;
+                bool all_idle = true;
+                for (auto& s : slots) all_idle = all_idle && s.phase == 0;
+                if (all_idle) return;
             }
-            if (busy)
+            if (gathering)
+                std::this_thread::yield();  // a timed wait would overshoot
+            else if (busy)
                 cv_sched.wait_for(lk, std::chrono::microseconds(50));
             else
                 cv_sched.wait_for(lk, std::chrono::milliseconds(5), [&] { return stop || !pending.empty(); });

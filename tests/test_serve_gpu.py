@@ -47,6 +47,22 @@ def test_budget_of_the_partitioned_join_is_enough(bj, oracle, torch_cuda, room):
             assert_same_pairs(oracle, a, b, er, es)
 
 
+def test_a_burst_of_small_requests_takes_two_waves(bj, torch_cuda):
+    """The first request of a burst starts at once; the other slot waits for the rest instead of taking the next
+    one or two, which would make the rest wait for a whole wave."""
+    n_r, n_s = 65_536, 262_144
+    d = [torch_cuda.empty(n, dtype=torch_cuda.int32, device="cuda") for n in (n_r, n_r, n_s, n_s)]
+    bj.gen_device(3, n_r, n_s, 0.1, 0.0, *d)
+    torch_cuda.cuda.synchronize()
+    waves = []
+    with bj.Server(use_bloom=1) as srv:
+        for _ in range(8):
+            res = [srv.poll(t)[0] for t in [srv.submit(*d, capacity=n_s // 8, on_device=True) for _ in range(12)]]
+            assert all(r.status == bj.BRIG_OK and r.count == n_s // 10 for r in res)
+            waves.append(len({r.wave for r in res}))
+    assert min(waves[2:]) <= 2, waves
+
+
 def test_same_result_alone_and_in_mix(bj, oracle, torch_cuda):
     x = _req(bj, 77, 150_000, 4, 0.5)
     er, es = oracle.pairs(*x)
