@@ -86,6 +86,37 @@ def test_batch_graph_replay_new_inputs(bj, oracle, torch_cuda):
                                   o_s[:c].cpu().numpy().view(np.uint32), er, es)
 
 
+def test_batch_graph_between_unpartitioned_joins(bj, oracle, torch_cuda):
+    """One handle's workspace and captured graph: a batch replayed after single joins that run unpartitioned in the
+    same workspace, one of which grows it."""
+    def inputs(*a):
+        data = bj.gen_host(*a)
+        return data, oracle.pairs(*data), [dev(torch_cuda, x) for x in data]
+
+    batch = [inputs(20 + i, n_r, n_s, 0.3) for i, (n_r, n_s) in enumerate([(30_000, 70_000), (1000, 5000)])]
+    small, large = inputs(30, 20_000, 30_000, 0.5), inputs(31, 1_500_000, 1_500_000, 0.2)
+    out = [torch_cuda.empty(400_000, dtype=torch_cuda.int32, device="cuda") for _ in range(4)]
+
+    def check(out_r, out_s, count, exp):
+        assert count == len(exp[0])
+        assert_same_pairs(oracle, out_r[:count].cpu().numpy().view(np.uint32), out_s[:count].cpu().numpy().view(np.uint32), *exp)
+
+    with bj.Join(use_cuda_graph=1) as j:
+        for step in (batch, batch, small, batch, large, batch, small, batch):
+            n0 = bj.kernel_launches()
+            if step is batch:
+                j.run_batch([dict(r_key=d[0], r_val=d[1], n_r=len(x[0]), s_key=d[2], s_val=d[3], n_s=len(x[2]),
+                                  out_r=out[2 * i], out_s=out[2 * i + 1], capacity=400_000)
+                             for i, (x, _, d) in enumerate(batch)])
+                for i, c in enumerate(j.batch_counts(2)):
+                    check(out[2 * i], out[2 * i + 1], int(c), batch[i][1])
+            else:
+                x, exp, d = step
+                j.run(d[0], d[1], len(x[0]), d[2], d[3], len(x[2]), out[0], out[1], 400_000)
+                check(out[0], out[1], j.stats().count, exp)
+            assert (bj.kernel_launches() - n0 == 1) == (step is not batch)
+
+
 def _skewed_cases(bj, oracle, n, seed):
     rng = np.random.default_rng(seed)
     cases, exps = [], []

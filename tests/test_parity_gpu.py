@@ -8,6 +8,25 @@ from gpu_helpers import assert_same_pairs, run_device
 pytestmark = pytest.mark.gpu
 
 
+# Small joins of a default configuration run unpartitioned, as one kernel; table_capacity=4096, the default
+# size, keeps the partitioned pipeline.
+both_paths = pytest.mark.parametrize("path", [dict(), dict(table_capacity=4096)], ids=["one_kernel", "partitioned"])
+
+
+class ran:
+    """The joins inside took the path."""
+
+    def __init__(self, bj, path):
+        self.bj, self.path = bj, path
+
+    def __enter__(self):
+        self.n0 = self.bj.kernel_launches()
+
+    def __exit__(self, kind, *_):
+        if kind is None:
+            assert (self.bj.kernel_launches() - self.n0 > 1) == bool(self.path)
+
+
 def _parity(bj, oracle, torch, rk, rv, sk, sv, cap=None, **cfg):
     exp_r, exp_s = oracle.pairs(rk, rv, sk, sv)
     st, r, s, _ = run_device(bj, torch, rk, rv, sk, sv, cap=cap if cap is not None else max(len(exp_r), 1), **cfg)
@@ -16,11 +35,13 @@ def _parity(bj, oracle, torch, rk, rv, sk, sv, cap=None, **cfg):
     return st
 
 
+@both_paths
 @pytest.mark.parametrize("bloom", [0, 1])
 @pytest.mark.parametrize("n", [1000, 100_000, 1 << 20])
-def test_uniform_hash(bj, oracle, torch_cuda, n, bloom):
+def test_uniform_hash(bj, oracle, torch_cuda, n, bloom, path):
     rk, rv, sk, sv = bj.gen_host(7 + n, n, n, 0.1)
-    st = _parity(bj, oracle, torch_cuda, rk, rv, sk, sv, use_bloom=bloom)
+    with ran(bj, path):
+        st = _parity(bj, oracle, torch_cuda, rk, rv, sk, sv, use_bloom=bloom, **path)
     assert st.count == n // 10
     if bloom:
         assert st.count <= st.s_survivors < n
@@ -112,15 +133,17 @@ def test_single_hot_key(bj, oracle, torch_cuda):
     assert st.count == 3000 * 700 and st.split_tasks > 0
 
 
+@both_paths
 @pytest.mark.parametrize("bloom", [0, 1])
-def test_edge_keys_full_domain(bj, oracle, torch_cuda, bloom):
+def test_edge_keys_full_domain(bj, oracle, torch_cuda, bloom, path):
     edge = np.array([0, 1, 0x7FFFFFFF, 0x80000000, 0x80000001, 0xFFFFFFFE, 0xFFFFFFFF], np.uint32)
     rng = np.random.default_rng(5)
     rk = np.concatenate([edge, edge, rng.integers(0, 2**32, 5000, dtype=np.uint64).astype(np.uint32)])
     sk = np.concatenate([edge, rng.permutation(rk)[:3000], rng.integers(0, 2**32, 3000, dtype=np.uint64).astype(np.uint32)])
     rv = rng.integers(0, 2**32, len(rk), dtype=np.uint64).astype(np.uint32)
     sv = rng.integers(0, 2**32, len(sk), dtype=np.uint64).astype(np.uint32)
-    _parity(bj, oracle, torch_cuda, rk, rv, sk, sv, use_bloom=bloom)
+    with ran(bj, path):
+        _parity(bj, oracle, torch_cuda, rk, rv, sk, sv, use_bloom=bloom, **path)
 
 
 @pytest.mark.parametrize("nr,ns", [(0, 100), (100, 0), (0, 0), (1, 1)])
@@ -131,40 +154,48 @@ def test_empty_and_tiny(bj, oracle, torch_cuda, nr, ns):
     assert st.count == min(nr, ns)
 
 
-def test_ragged_unaligned_inputs(bj, oracle, torch_cuda):
+@both_paths
+def test_ragged_unaligned_inputs(bj, oracle, torch_cuda, path):
     rk, rv, sk, sv = bj.gen_host(21, 99_999, 77_777, 0.5)
     exp_r, exp_s = oracle.pairs(rk, rv, sk, sv)
-    st, r, s, _ = run_device(bj, torch_cuda, rk, rv, sk, sv, cap=len(exp_r), offset=1, use_bloom=1)
+    with ran(bj, path):
+        st, r, s, _ = run_device(bj, torch_cuda, rk, rv, sk, sv, cap=len(exp_r), offset=1, use_bloom=1, **path)
     assert st.count == len(exp_r)
     assert_same_pairs(oracle, r, s, exp_r, exp_s)
 
 
+@both_paths
 @pytest.mark.parametrize("offsets", [(1, 3, 2, 0), (3, 1, 0, 2), (2, 2, 3, 1)])
 @pytest.mark.parametrize("mode", [0, 1])
-def test_differently_misaligned_key_and_value_arrays(bj, oracle, torch_cuda, offsets, mode):
+def test_differently_misaligned_key_and_value_arrays(bj, oracle, torch_cuda, offsets, mode, path):
     # keys and values misaligned by different amounts, over many scatter tiles per slice
     rk, rv, sk, sv = bj.gen_host(31, 700_001, 900_003, 0.2)
     exp_r, exp_s = oracle.pairs(rk, rv, sk, sv)
-    st, r, s, _ = run_device(bj, torch_cuda, rk, rv, sk, sv, cap=len(exp_r), offset=offsets,
-                             partition_mode=mode, use_bloom=mode)
+    with ran(bj, path):
+        st, r, s, _ = run_device(bj, torch_cuda, rk, rv, sk, sv, cap=len(exp_r), offset=offsets,
+                                 partition_mode=mode, use_bloom=mode, **path)
     assert st.count == len(exp_r)
     assert_same_pairs(oracle, r, s, exp_r, exp_s)
 
 
-def test_capacity_overflow_counts_exactly(bj, oracle, torch_cuda):
+@both_paths
+def test_capacity_overflow_counts_exactly(bj, oracle, torch_cuda, path):
     rk, rv, sk, sv = bj.gen_host(3, 50_000, 50_000, 0.4)
     exp_r, exp_s = oracle.pairs(rk, rv, sk, sv)
     cap = len(exp_r) // 3
-    st, r, s, _ = run_device(bj, torch_cuda, rk, rv, sk, sv, cap=cap)
+    with ran(bj, path):
+        st, r, s, _ = run_device(bj, torch_cuda, rk, rv, sk, sv, cap=cap, **path)
     assert st.count == len(exp_r) and st.overflow == 1 and st.written == cap and len(r) == cap
     exp = set(zip(exp_r.tolist(), exp_s.tolist()))
     got = list(zip(r.tolist(), s.tolist()))
     assert len(set(got)) == cap and all(p in exp for p in got)
 
 
-def test_emit_key(bj, oracle, torch_cuda):
+@both_paths
+def test_emit_key(bj, oracle, torch_cuda, path):
     rk, rv, sk, sv = bj.gen_host(4, 30_000, 40_000, 0.2)
-    st, r, s, k = run_device(bj, torch_cuda, rk, rv, sk, sv, emit_key=True)
+    with ran(bj, path):
+        st, r, s, k = run_device(bj, torch_cuda, rk, rv, sk, sv, emit_key=True, **path)
     assert np.array_equal(k, rk[r]) and np.array_equal(k, sk[s])
 
 
@@ -192,20 +223,23 @@ def test_long_and_short_buckets_in_one_warp(bj, oracle, torch_cuda, build_side):
         _parity(bj, oracle, torch_cuda, rk, rv, sk, sv, use_bloom=bloom, table_capacity=1024, emit_key=True)
 
 
-def test_handle_reuse_and_graph_replay(bj, oracle, torch_cuda):
-    with bj.Join(use_bloom=1, use_cuda_graph=1) as j:
+@both_paths
+def test_handle_reuse_and_graph_replay(bj, oracle, torch_cuda, path):
+    with bj.Join(use_bloom=1, use_cuda_graph=1, **path) as j:
         for seed in (1, 2, 3):
             rk, rv, sk, sv = bj.gen_host(seed, 120_000, 90_000, 0.25)
             exp_r, exp_s = oracle.pairs(rk, rv, sk, sv)
-            st, r, s, _ = run_device(bj, torch_cuda, rk, rv, sk, sv, cap=len(exp_r) + 10, handle=j)
+            with ran(bj, path):
+                st, r, s, _ = run_device(bj, torch_cuda, rk, rv, sk, sv, cap=len(exp_r) + 10, handle=j)
             assert st.count == len(exp_r)
             assert_same_pairs(oracle, r, s, exp_r, exp_s)
 
 
-def test_run_host_entry_point(bj, oracle):
+@both_paths
+def test_run_host_entry_point(bj, oracle, path):
     rk, rv, sk, sv = bj.gen_host(8, 70_000, 60_000, 0.3)
     exp_r, exp_s = oracle.pairs(rk, rv, sk, sv)
-    with bj.Join(use_bloom=1) as j:
+    with bj.Join(use_bloom=1, **path) as j, ran(bj, path):
         cnt, r, s = j.run_host(rk, rv, sk, sv, capacity=len(exp_r))
     assert cnt == len(exp_r)
     assert_same_pairs(oracle, r, s, exp_r, exp_s)
@@ -345,16 +379,18 @@ def test_gather_rate_helper(bj, torch_cuda):
         bj.gather_rate(table[:1000], 1 << 20, sink)
 
 
-def test_adaptive_bloom_switches_off_and_retests(bj, oracle, torch_cuda):
+@both_paths
+def test_adaptive_bloom_switches_off_and_retests(bj, oracle, torch_cuda, path):
     """use_bloom = BLOOM_ADAPTIVE: a run whose filter lets more than 30% of S through turns the filter
     off for the handle's next single joins, every 16th of which tests it again; once a test run
     sees few survivors the filter stays on. Every run is exact."""
     hi = bj.gen_host(71, 200_000, 300_000, 0.6)   # 60% of S matches: the filter does not pay
     lo = bj.gen_host(72, 200_000, 300_000, 0.05)  # 5% matches: it does
     exp = {id(x): oracle.pairs(*x) for x in (hi, lo)}
-    with bj.Join(use_bloom=bj.BLOOM_ADAPTIVE) as j:
+    with bj.Join(use_bloom=bj.BLOOM_ADAPTIVE, **path) as j:
         def run(data):
-            st, r, s, _ = run_device(bj, torch_cuda, *data, cap=len(data[2]), handle=j)
+            with ran(bj, path):
+                st, r, s, _ = run_device(bj, torch_cuda, *data, cap=len(data[2]), handle=j)
             er, es = exp[id(data)]
             assert st.count == len(er)
             assert_same_pairs(oracle, r, s, er, es)
