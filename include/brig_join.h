@@ -110,7 +110,8 @@ typedef struct brig_join_config {
                                        of the partition passes); 0 = 4 for one join, 16 for a batch */
 } brig_join_config;
 
-/* Output of one join. Pairs are written in an unspecified order; the multiset is exact. When the
+/* Output of one join. Pairs are written in an unspecified order; the multiset is exact. The arrays may
+ * share memory with the join's inputs, which are then overwritten. When the
  * number of matches exceeds `capacity`, the first `capacity` reserved slots are written, the count
  * stays exact and the run reports BRIG_E_OVERFLOW through brig_join_get_stats (the reference
  * writes only below d_answer_capacity, src/kernel_functions.cu:421, and counts all matches). */
