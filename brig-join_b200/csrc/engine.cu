@@ -439,12 +439,15 @@ void Engine::ensure_host_io(int64_t nr, int64_t ns, int64_t cap, bool key) {
 }
 
 // Waits for the work that a run has enqueued when the run fails before its end: nothing marks that work for the
-// handle's next run or its destruction, which free the workspace it uses.
+// handle's next run or its destruction, which free the workspace it uses, or for the caller, whose host arrays
+// the copies on `copies` (may be null) read.
 struct FailedRunWait {
-    cudaStream_t stream;
+    cudaStream_t stream, copies;
     bool done = false;
     ~FailedRunWait() {
-        if (!done) cudaStreamSynchronize(stream);
+        if (done) return;
+        cudaStreamSynchronize(stream);
+        if (copies) cudaStreamSynchronize(copies);
     }
 };
 
@@ -489,7 +492,7 @@ void Engine::run_host_chunked(const uint32_t* rk, const uint32_t* rv, int64_t nr
                    "descriptor upload");
         cuda_check(enqueue_pipeline(a, st), "pipeline launch");
     };
-    FailedRunWait wait{st};
+    FailedRunWait wait{st, copy_stream};
     // R: copied once, then its two passes and the Bloom build
     cuda_check(cudaMemcpyAsync(hio.rk, rk, (size_t)nr * 4, cudaMemcpyHostToDevice, st), "H2D R keys");
     cuda_check(cudaMemcpyAsync(hio.rv, rv, (size_t)nr * 4, cudaMemcpyHostToDevice, st), "H2D R vals");
@@ -761,7 +764,7 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
         ns[j] = joins[j].ns;
     }
     std::vector<JoinPlan> plans = plan_batch(adapt_config(nj), nr.data(), ns.data(), nj, shared_l2_);
-    FailedRunWait wait{stream};
+    FailedRunWait wait{stream, s_ready ? copy_stream : nullptr};
     bool direct = nj == 1 && direct_eligible(cfg_, plans[0], joins[0].out.capacity) && !writes_inputs(joins[0]);
     // While S is still being copied from the host, the partitioned join works on R; the direct join is one
     // kernel that starts after the copy.
