@@ -762,8 +762,8 @@ __device__ __forceinline__ void probe_queued(const Ctx& c, const DirectJoin& d, 
 // the last one is worked off. Few values live across the two parts: with a step's table entries held
 // beside its rows, 64 registers spilled, and two CTAs' spills do not fit L1 (16.8M rows, 2M-tuple table:
 // 322 us). Of the 230 to 250 bytes of spill stores that remain, all but 12 to 28 save registers across the
-// calls out of line (flush_staged, probe_rest, probe_long), which few warps' steps make. kFilter: rows are tested against the filter first (S of a fused join). Returns this lane's
-// rows that passed.
+// calls out of line (flush_staged, probe_rest, probe_long), which few warps' steps make. kFilter: rows are
+// tested against the filter first (S of a fused join). Returns this lane's rows that passed.
 template <bool kPacked, bool kFilter, int M, int K>
 __device__ __noinline__ uint32_t probe_run(const Ctx& c, const DirectJoin& d, const Role& r, int rel,
                                            uint32_t row0, uint32_t n, const uint2* pat) {

@@ -763,7 +763,8 @@ k_l1_hist(const JoinDesc* __restrict__ J, int nj, int rel, const int64_t* __rest
                 // and turn. A lane has few, so a warp takes about two turns; going through the six keys in
                 // order ran nearly six, each for a few lanes (16.8M keys, 21 MB filter, 12% surviving: 145 us
                 // against 108; 1G keys, 84 MB filter, 3%: 5.94 ms against 5.83: there the filter's reads bind,
-                // 13 of the 19 cycles between a warp's instructions). The level-2 pass, four keys a group, was slower this way (3.07 to 3.23 ms at 640M).
+                // 13 of the 19 cycles between a warp's instructions). The level-2 pass, four keys a group, was
+                // slower this way (3.07 to 3.23 ms at 640M).
                 const uint32_t tot = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(pm));
                 if (tot) {
                     uint32_t base = 0;
