@@ -32,8 +32,8 @@ using Clock = std::chrono::steady_clock;
 // for kQuiet, or kGather after the launch before it. A lone request's join takes the host 8 us to launch, and
 // without this the first three of a burst took both slots and the rest often waited for a whole wave. First submit
 // to last result in us, median / 90th percentile of 200 bursts (with it; without; when every launch took the host
-// 0.1 ms): 12 requests of 65K x 262K 541 / 557; 527 / 664 to 815; 557 / 565. 6 of 262K x 1M 508 / 517; 510 / 720,
-// in one process of three 776 / 786; 537 / 544. A caller that works on the first answers while it waits for the
+// 0.1 ms): 12 requests of 65K x 262K 541 / 557; 527 / 664 to 815; 557 / 565. 6 of 262K x 1M 509 / 517; 510 / 525 to
+// 722, in one process of three 776 / 786; 537 / 544. A caller that works on the first answers while it waits for the
 // rest has fewer to start with: 12 requests of 65K to 1M rows with their pairs placed on the host 1.66 to 1.69 ms
 // with it, 1.61 to 1.67 without. Meanwhile the scheduler looks every kLook and leaves the lock to the submitters:
 // looking all the time held them up, so that the burst came in three waves (16 requests of up to 524K rows: 1.13 ms
