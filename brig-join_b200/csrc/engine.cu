@@ -18,6 +18,7 @@ namespace brig {
 
 void cuda_check(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return;
+    cudaGetLastError();  // reported here: not again by the next launch's check
     const int st = (e == cudaErrorMemoryAllocation) ? BRIG_E_NOMEM : BRIG_E_CUDA;
     fail(st, std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -448,6 +449,7 @@ struct FailedRunWait {
         if (done) return;
         cudaStreamSynchronize(stream);
         if (copies) cudaStreamSynchronize(copies);
+        cudaGetLastError();
     }
 };
 
@@ -723,6 +725,13 @@ static bool writes_inputs(const JoinIO& io) {
     return false;
 }
 
+static bool is_capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus st;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 bool Engine::run_direct(const std::vector<JoinIO>& joins, const std::vector<JoinPlan>& plans, cudaStream_t stream) {
     const JoinPlan& p = plans[0];
     int& per_sm = direct_ctas_[!p.bloom ? 0 : 1 + 2 * (p.pf.mode != 0) + (p.k == kBloomFastK)];
@@ -769,6 +778,10 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
     // While S is still being copied from the host, the partitioned join works on R; the direct join is one
     // kernel that starts after the copy.
     if (s_ready) direct = direct && std::min(nr[0], ns[0]) <= (nr[0] > ns[0] ? kDirectMaxLateR : kDirectMaxLateS);
+    // A caller's capture refuses the partitioned join (a first run by its pinned staging buffer, a later one by
+    // the wait for the run before). The direct join's first run would be captured: with a workspace that only the
+    // captured graph owns, and an end that no later call can wait for.
+    if (direct && !have_run_) direct = !is_capturing(stream);
     // A direct join's descriptor is its kernel's argument, so a graph would save it nothing.
     if (direct) {
         if (s_ready) cuda_check(cudaStreamWaitEvent(stream, s_ready, 0), "cudaStreamWaitEvent");
@@ -780,8 +793,8 @@ void Engine::run(const std::vector<JoinIO>& joins, cudaStream_t stream, bool use
     // A handle's runs are ordered even across streams: this run's work (and a workspace growth)
     // starts after the previous run's last operation.
     if (have_run_) cuda_check(cudaStreamWaitEvent(stream, done_, 0), "cudaStreamWaitEvent");
+    ensure_staging(sh.meta_bytes);  // first: under capture it fails, and a workspace would be the graph's
     ensure_workspace(sh.total, stream);
-    ensure_staging(sh.meta_bytes);
     // The staging buffer may still be read by the previous run's copy.
     if (have_run_) cuda_check(cudaEventSynchronize(stage_free_), "cudaEventSynchronize");
 

@@ -1,5 +1,6 @@
 """The unpartitioned join (one cooperative kernel) against the oracle and the partitioned join: step and
 tile remainders, both build sides, long buckets, the limits of the rule that chooses it."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -209,3 +210,28 @@ def test_misaligned_overflow_and_reuse(bj, oracle, torch_cuda):
                 assert_same_pairs(oracle, r, s, *exp)
             else:
                 assert set(zip(r.tolist(), s.tolist())) <= set(zip(exp[0].tolist(), exp[1].tolist()))
+
+
+@pytest.mark.parametrize("path", [dict(), dict(table_capacity=4096)], ids=["default", "partitioned"])
+def test_a_captured_run_is_refused(bj, oracle, torch_cuda, path):
+    """Under a caller's stream capture no run is taken, and the handle runs again after it."""
+    torch, cu = torch_cuda, ctypes.CDLL("libcuda.so.1")
+    data = bj.gen_host(3, 5000, 9000, 0.4)
+    exp = oracle.pairs(*data)
+    d = [torch.from_numpy(x.view(np.int32)).cuda() for x in data]
+    out = [torch.empty(len(exp[0]), dtype=torch.int32, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    with bj.Join(**path) as j:
+        for _ in range(2):  # a handle's first run, and one after another
+            stream, graph = torch.cuda.Stream(), ctypes.c_void_p()
+            h = ctypes.c_void_p(stream.cuda_stream)
+            assert cu.cuStreamBeginCapture_v2(h, 0) == 0  # CU_STREAM_CAPTURE_MODE_GLOBAL
+            try:
+                with pytest.raises(bj.BrigError):
+                    j.run(d[0], d[1], 5000, d[2], d[3], 9000, *out, len(exp[0]), stream=stream.cuda_stream)
+            finally:
+                if cu.cuStreamEndCapture(h, ctypes.byref(graph)) == 0 and graph:
+                    cu.cuGraphDestroy(graph)
+            st, r, s, _ = run_device(bj, torch, *data, cap=len(exp[0]), handle=j)
+            assert st.count == len(exp[0])
+            assert_same_pairs(oracle, r, s, *exp)
