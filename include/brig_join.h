@@ -161,7 +161,11 @@ int brig_join_destroy(brig_join_t* h);
  * partial_jointable_gpu_partition_r_only (src/vlsplit_hash_kernel.cu:224-255), the partitioned
  * Bloom build (src/hash_kernel.cu:670-705), queryAndCompactKernelPartitioned
  * (src/bloom.cu:725-773), partial_jointable_gpu_partition_s_only (src/vlsplit_hash_kernel.cu:258-297)
- * and join_execute_host (src/join_executor.cu:14-515). n_r or n_s may be 0. */
+ * and join_execute_host (src/join_executor.cu:14-515). n_r or n_s may be 0.
+ * A small join of a handle that leaves its sizes to the planner is one cooperative launch, which starts when
+ * all its CTAs fit on the GPU together. A program that keeps another kernel on the GPU until the join has
+ * finished (a resident kernel that waits for the pairs, a receive posted before the join whose peer waits for
+ * them) sets table_capacity (4096 is the default size): its joins then run partitioned, in ordinary launches. */
 int brig_join_run(brig_join_t* h,
                   const uint32_t* r_key, const uint32_t* r_val, int64_t n_r,
                   const uint32_t* s_key, const uint32_t* s_val, int64_t n_s,
